@@ -46,3 +46,26 @@ def test_gdn_chunk_kernels_match_torch_chunked_form(V):
     assert (A - A_r).abs().max().item() < 2e-2 * max(1.0, A_r.abs().max().item())
     assert (o.float() - o_r).abs().max().item() < 2e-2 * (o_r.abs().max().item() + 1e-6)
     assert (ht - ht_r).abs().max().item() < 2e-2 * (ht_r.abs().max().item() + 1e-6)
+
+
+@pytest.mark.parametrize("H,V,lens", [(2, 64, [1]), (2, 64, [64, 128]), (3, 192, [63, 65, 0, 130]), (2, 256, [0, 200, 17, 0]),
+                                      (16, 128, [70]), (16, 128, [66, 129]), (16, 256, [5, 64, 100])])
+def test_gdn_chunk_kernels_over_column_tiles_and_sequence_ends(H, V, lens):
+    """Every width of the state walk (16 columns alone on an SM, 16 columns two to an SM, 32 columns), empty sequences, full and ragged
+    last chunks.  Tolerance: operands of the products are bf16 (2^-9 relative), a result is a sum of a few of them."""
+    from test_gdn_cpu import _inputs
+    from triton_distributed_b200 import ops
+
+    K, T = 128, sum(lens)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    q, k, v, g, beta = _inputs(T, H, K, V, seed=11, dtype=torch.bfloat16, device="cuda")
+    h0 = torch.randn(len(lens), H, K, V, device="cuda") * 0.1
+    gc, o, A, ht = ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, h0, True, cu, return_A=True, impl="chunk")
+    o_r, s_r = ops.gated_delta_rule_recurrent(q, k, v, g, beta, K ** -0.5, h0, cu)
+    cum = torch.cat([g[0, t:min(t + 64, b)].double().cumsum(0) for a, b in zip(cu.tolist(), cu.tolist()[1:]) for t in range(a, b, 64)])
+    torch.testing.assert_close(gc[0].double(), cum, rtol=1e-5, atol=1e-5)
+    assert (A.triu(1) if T == 1 else A)[0, 0, 0, 1:].abs().max().item() == 0.0
+    assert (o.float() - o_r).norm().item() < 2 ** -7 * o_r.norm().item()
+    assert (ht - s_r).norm().item() < 2 ** -7 * s_r.norm().item()
+    empty = [i for i, n in enumerate(lens) if n == 0]
+    assert torch.equal(ht[empty], h0[empty])

@@ -34,12 +34,9 @@ using attn::mma_bf16;
 using namespace chunk;
 
 constexpr int kThreads = 256;
-constexpr int kFp = kC + 4;       // pitch of fp32 [64][64] matrices
 constexpr int kSp = kC + 8;       // pitch of bf16 [64][64] slabs
 
 // ---------------------------------------------------------------------------------------------------- chunk-local matrices
-// Lower 16 x 16 block (bi, bj) of a 64 x 64 matrix.
-TDB_DEVICE constexpr int lower_block(int bi, int bj) { return bi * (bi + 1) / 2 + bj; }
 constexpr int kFrags = 10 * 64;    // uint4 of a lower triangular matrix as A fragments: ten blocks, high and low parts of 32 lanes
 
 struct LocalSmem {
@@ -106,62 +103,6 @@ TDB_DEVICE void store_a_fragment(uint4* dst, const float (&a)[4], const float (&
   const HiLo r0 = split2(a[0], a[1]), r1 = split2(a[2], a[3]), r2 = split2(b[0], b[1]), r3 = split2(b[2], b[3]);
   dst[0] = make_uint4(r0.hi, r1.hi, r2.hi, r3.hi);
   dst[32] = make_uint4(r0.lo, r1.lo, r2.lo, r3.lo);
-}
-
-// A <- (I + A)^-1 for the strictly lower triangular A (blocks above the diagonal are scratch).
-TDB_DEVICE void invert_unit_lower(float* A) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp < 4) {                       // the 16 x 16 blocks on the diagonal by substitution, a column per lane
-    float* D = A + (warp * 16) * kFp + warp * 16;
-    float x[16];
-    const int j = lane & 15;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float a = (i == j) ? 1.f : 0.f, b = 0.f;
-#pragma unroll
-      for (int m = 0; m < i; ++m) {
-        if (m & 1) a = fmaf(-D[i * kFp + m], x[m], a);
-        else b = fmaf(-D[i * kFp + m], x[m], b);
-      }
-      x[i] = a + b;
-    }
-    __syncwarp();
-    if (lane < 16) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) D[i * kFp + j] = i >= j ? x[i] : 0.f;
-    }
-  }
-  __syncthreads();
-  // blocks below the diagonal, 16 then 32: A21 = -A22 (L21 A11); the product in brackets goes to the block above the diagonal.
-  // A thread owns four neighbouring columns of a row.
-#pragma unroll
-  for (int n = 16; n <= 32; n *= 2) {
-    const int per = n * n / 4, all = 32 / n * per;
-    for (int i = tid; i < all; i += kThreads) {
-      const int b = (i / per) * 2 * n, r = (i % per) / (n / 4), c = (i % (n / 4)) * 4;
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-      for (int m = c & ~15; m < n; ++m) {
-        const float l = A[(b + n + r) * kFp + b + m];
-        const float4 v = *reinterpret_cast<const float4*>(A + (b + m) * kFp + b + c);
-        a.x = fmaf(l, v.x, a.x); a.y = fmaf(l, v.y, a.y); a.z = fmaf(l, v.z, a.z); a.w = fmaf(l, v.w, a.w);
-      }
-      *reinterpret_cast<float4*>(A + (b + r) * kFp + b + n + c) = a;
-    }
-    __syncthreads();
-    for (int i = tid; i < all; i += kThreads) {
-      const int b = (i / per) * 2 * n, r = (i % per) / (n / 4), c = (i % (n / 4)) * 4;
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-      for (int m = 0; m < (r & ~15) + 16; ++m) {
-        const float l = -A[(b + n + r) * kFp + b + n + m];
-        const float4 v = *reinterpret_cast<const float4*>(A + (b + m) * kFp + b + n + c);
-        a.x = fmaf(l, v.x, a.x); a.y = fmaf(l, v.y, a.y); a.z = fmaf(l, v.z, a.z); a.w = fmaf(l, v.w, a.w);
-      }
-      *reinterpret_cast<float4*>(A + (b + n + r) * kFp + b + c) = a;
-    }
-    __syncthreads();
-  }
 }
 
 // Fragments of A beta and A beta e^{gc} take the place of A.
@@ -293,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 2) delta_local_kernel(const DeltaArg
   __syncthreads();                      // Q is no longer needed: its place takes the slabs
   load_tile(s.vs, kSp, v_g, Hv, min(64, p.dv), cp.n, kThreads);
   cp_async_commit();
-  invert_unit_lower(s.A);
+  invert_unit_lower<kThreads>(s.A);
   split_inverse(s);
 
   const int64_t ch = static_cast<int64_t>(chunk) * p.H + h;

@@ -3,28 +3,34 @@
 // Per chunk (rows i, j of one chunk, gc = chunk-local cumulative log decay):
 //     L[i][j] = beta_i (k_i . k_j) exp(gc_i - gc_j)        for i > j, else 0
 //     A       = (I + L)^-1                                  (unit lower triangular)
-//     w       = A (beta k exp(gc)),   u = A (beta v)
+//     w       = A (beta k exp(gc)),   u = A (beta v),       kd = k exp(gc_last - gc)
 // then, sequentially over the chunks of a sequence with the state S [K x V] at the start of the chunk:
 //     v_new   = u - w S
-//     S      <- S exp(gc_last) + (k exp(gc_last - gc))^T v_new
+//     S      <- S exp(gc_last) + kd^T v_new
 // and per chunk again:
-//     o       = scale [ (q exp(gc)) S + tril(q k^T exp(gc_i - gc_j)) v_new ]
+//     o       = scale [ exp(gc) (q S) + tril(q k^T exp(gc_i - gc_j)) v_new ]
 //
-// Three kernels, as in the reference (python/triton_dist/kernels/nvidia/gdn.py:123 scaled-dot KK^T + :300 solve +
-// :482 recompute w/u, :620 chunk state pass, :785 output; entry point :926):
-//   gdn_chunk_prepare   grid (chunks, H): KK^T on tensor cores, forward substitution in shared memory, w / u on tensor cores
-//   gdn_chunk_state     grid (V / 64, H, sequences): walks the chunks with S in shared memory (fp32), two tensor-core
-//                       products per chunk; writes v_new and the chunk-start states (bf16)
-//   gdn_chunk_output    grid (chunks, H, V / 64): q k^T, masking / decay, two tensor-core products
-// Tensor-core products use the warp-level bf16 MMA (fragments through nvcuda::wmma, fp32 accumulation): 64 x 64 x 128
-// problems are too small for a tcgen05 / TMEM pipeline to pay.  Intermediates (w, u, v_new) live in a chunk-major layout
-// [chunk][H][64][*] whose padded rows are zero, so no kernel reads past a sequence end.
+// The mathematics of the reference (python/triton_dist/kernels/nvidia/gdn.py:123 scaled-dot KK^T, :300 solve, :482 recompute
+// w / u, :620 chunk state pass, :785 output; entry point :926).  Four launches, chained with programmatic dependent launch:
+//   gdn_chunk_tables    one CTA: which chunk belongs to which sequence.  cu_seqlens is a device tensor; reading it on the host
+//                       would make every call wait for the stream.
+//   gdn_chunk_prepare   grid (chunks, H): KK^T, triangular inverse, w / u / kd
+//   gdn_chunk_state     grid (V / 16 or V / 32, H, sequences): walks the chunks, S in fp32 registers
+//   gdn_chunk_output    grid (chunks, H): q k^T, decay, two products
+// Products use the warp-level bf16 MMA: 64 x 64 x 128 problems in a serial chain are too small for a tcgen05 / TMEM pipeline.
+// What travels between the kernels (w, kd, u, v_new and S in bf16, as the tensor cores take them) is stored in the order in which
+// the lanes of a warp hold the fragments of m16n8k16, so that every load is 16 coalesced bytes per lane and nothing is
+// rearranged in the serial kernel.  Rows beyond the end of a sequence are zero.
+//
+// Bound by the state walk, a chain of dependent chunks.  One sequence of 8192 tokens, 16 heads, V = 128 (B200): with S in shared
+// memory, 64 columns per CTA (32 CTAs) and row-major operands it took 6.5 us a chunk, now 0.95 us; the whole call 1606 -> 238 us
+// (prepare 374 -> 65 us through the blocked inverse on all threads, output 292 -> 51 us, and no wait for the stream).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <mma.h>
 
 #include <cstdint>
 
+#include "tdb/chunk.cuh"
 #include "tdb/gdn.h"
 #include "tdb/launch.cuh"
 
@@ -32,21 +38,21 @@ namespace tdb {
 
 namespace {
 
-using namespace nvcuda;
+using attn::cp_async16;
+using attn::cp_async_commit;
+using attn::cp_async_wait;
+using attn::ldmatrix_x4_trans;
+using attn::mma_bf16;
+using namespace chunk;
 
-constexpr int kC = 64;            // chunk length
-constexpr int kK = 128;           // head dim of q / k
-constexpr int kVT = 64;           // V columns per CTA in the state / output kernels
-constexpr int kThreads = 128;     // four warps, each owns 16 chunk rows
-constexpr int kLdK = kK + 8;      // bf16 row pitch of [64][128] tiles (272 bytes: 32-byte aligned 16-row tiles, no bank conflicts)
-constexpr int kLdC = kC + 8;      // bf16 row pitch of [*][64] tiles
-constexpr int kLdF = kC + 4;      // fp32 row pitch of [*][64] tiles
-
-using FragA = wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major>;
-using FragAT = wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::col_major>;
-using FragB = wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::row_major>;
-using FragBT = wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::col_major>;
-using FragC = wmma::fragment<wmma::accumulator, 16, 16, 16, float>;
+constexpr int kK = 128;            // head dim of q / k
+constexpr int kKs = kK / 16;       // k-steps of a product over it
+constexpr int kThreads = 256;      // prepare and output
+constexpr int kLdK = kK + 8;       // bf16 row pitch of [64][128] tiles (272 bytes: ldmatrix without bank conflicts)
+constexpr int kBlocks = 10;        // 16 x 16 blocks on and below the diagonal
+constexpr int kWFrag = 4 * kKs * 32;       // uint4 of w and of kd per (chunk, head)
+constexpr int kUFrag = 4 * 32;             // uint4 of u / v_new per 16 columns
+constexpr int kSFrag = kKs * 32;           // uint4 of S per 16 columns
 
 struct ChunkParams {
   const __nv_bfloat16* q;       // [T, H, K]
@@ -54,38 +60,101 @@ struct ChunkParams {
   const __nv_bfloat16* v;       // [T, H, V]
   const float* g;               // [T, H]
   const __nv_bfloat16* beta;    // [T, H]
-  const int32_t* cu_seqlens;    // [N + 1]
-  const int32_t* chunk_seq;     // [NC] sequence of every chunk
-  const int32_t* chunk_t0;      // [NC] first token of every chunk
-  const int32_t* seq_chunk0;    // [N + 1] first chunk of every sequence
+  const int32_t* cu;            // [N + 1]
+  int32_t* chunk_seq;           // [NC] sequence of every chunk
+  int32_t* chunk_t0;            // [NC] first token of every chunk
+  int32_t* seq_chunk0;          // [N + 1] first chunk of every sequence
   float* gcum;                  // [T, H] chunk-local cumulative log decay
   float* a_out;                 // [T, H, 64] or null
-  __nv_bfloat16* w;             // [NC, H, 64, K]
-  __nv_bfloat16* u;             // [NC, H, 64, V]
-  __nv_bfloat16* vnew;          // [NC, H, 64, V]
-  __nv_bfloat16* hstate;        // [NC, H, K, V] state at the start of every chunk
+  float* decay;                 // [NC, H] exp(gc_last)
+  uint4* w;                     // [NC, H, 4 row blocks, 8 k-steps, 32]     A fragments
+  uint4* kd;                    // [NC, H, 8 row blocks of K, 4 k-steps, 32] A fragments of kd^T
+  uint4* u;                     // [NC, H, V / 16, 4 row blocks, 32]        accumulator fragments of two 8-column tiles
+  uint4* vnew;                  // [NC, H, V / 16, 4 k-steps, 32]           B fragments of two 8-column tiles
+  uint4* hstate;                // [NC, H, V / 16, 8 k-steps, 32]           S at the start of the chunk, B fragments
   const float* h0;              // [N, H, K, V] or null
   float* ht;                    // [N, H, K, V] or null
   __nv_bfloat16* o;             // [T, H, V]
-  int H, V, NC;
+  int H, V, N, NC;              // NC: room in the tables, at least the number of chunks
   float scale;
 };
 
-__device__ __forceinline__ int chunk_len(const ChunkParams& p, int c) {
-  const int t0 = p.chunk_t0[c];
-  const int t_end = p.cu_seqlens[p.chunk_seq[c] + 1];
-  return min(kC, t_end - t0);
+// ------------------------------------------------------------------------------------------------------------------
+// Kernel 0: chunk tables
+// ------------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(kThreads) gdn_chunk_tables(const ChunkParams p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (warp == 0) {
+    int base = 0;
+    for (int s0 = 0; s0 < p.N; s0 += 32) {
+      const int s = s0 + lane;
+      const int own = s < p.N ? (max(p.cu[s + 1] - p.cu[s], 0) + kC - 1) / kC : 0;
+      int pre = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += x;
+      }
+      if (s < p.N) p.seq_chunk0[s] = min(base + pre - own, p.NC);
+      base += __shfl_sync(0xffffffffu, pre, 31);
+    }
+    if (lane == 0) p.seq_chunk0[p.N] = min(base, p.NC);
+  }
+  __syncthreads();
+  for (int s = warp; s < p.N; s += kThreads / 32) {
+    const int c0 = p.seq_chunk0[s], c1 = p.seq_chunk0[s + 1], t0 = p.cu[s];
+    for (int c = c0 + lane; c < c1; c += 32) {
+      p.chunk_seq[c] = s;
+      p.chunk_t0[c] = t0 + (c - c0) * kC;
+    }
+  }
 }
 
-// rows [0, n) of a token-major [T, H, cols] tensor into a padded shared tile, zero beyond n
-__device__ __forceinline__ void load_rows(__nv_bfloat16* dst, int ld, const __nv_bfloat16* src, int64_t t0, int n, int H, int h,
-                                          int cols, int col0, int ncols) {
-  const int vec = ncols / 8;
-  for (int i = threadIdx.x; i < kC * vec; i += kThreads) {
-    const int r = i / vec, c = (i - r * vec) * 8;
-    uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    if (r < n) val = *reinterpret_cast<const uint4*>(src + ((t0 + r) * H + h) * cols + col0 + c);
-    *reinterpret_cast<uint4*>(dst + r * ld + c) = val;
+// Two neighbouring accumulator tiles as one A fragment (also the form in which u travels).
+TDB_DEVICE uint4 pack_tiles(const float (&a)[4], const float (&b)[4]) {
+  return make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(b[0], b[1]), pack_bf16x2(b[2], b[3]));
+}
+TDB_DEVICE void zero(float (&a)[4]) { a[0] = a[1] = a[2] = a[3] = 0.f; }
+TDB_DEVICE int block_row(int i) { return i < 1 ? 0 : i < 3 ? 1 : i < 6 ? 2 : 3; }
+
+// 16 x 16 block (bi, bj) of X K^T, both [64][kLdK] in shared memory: two tiles of eight columns.
+TDB_DEVICE void score_block(const __nv_bfloat16* x, const __nv_bfloat16* k, int bi, int bj, float (&acc)[2][4]) {
+  const int lane = threadIdx.x & 31, mat = lane >> 3, mr = lane & 7;
+  const __nv_bfloat16* a0 = x + (bi * 16 + (mat & 1) * 8 + mr) * kLdK + (mat >> 1) * 8;
+  const __nv_bfloat16* b0 = k + (bj * 16 + (mat >> 1) * 8 + mr) * kLdK + (mat & 1) * 8;
+  zero(acc[0]);
+  zero(acc[1]);
+#pragma unroll
+  for (int ks = 0; ks < kKs; ++ks) {
+    uint32_t a[4], b[4];
+    ldmatrix_x4(a, a0 + ks * 16);
+    ldmatrix_x4(b, b0 + ks * 16);
+    mma_bf16(acc[0], a, b[0], b[1]);
+    mma_bf16(acc[1], a, b[2], b[3]);
+  }
+}
+
+// Four row blocks of (lower triangular X as fragments) x (64 tokens x 16 columns at b0 in shared memory).
+TDB_DEVICE void lower_times(float (&acc)[4][2][4], const uint4* xf, const __nv_bfloat16* b0, int pitch) {
+  const int lane = threadIdx.x & 31, mat = lane >> 3, mr = lane & 7;
+#pragma unroll
+  for (int rb = 0; rb < 4; ++rb) {
+    zero(acc[rb][0]);
+    zero(acc[rb][1]);
+  }
+#pragma unroll
+  for (int kb = 0; kb < 4; ++kb) {
+    uint32_t b[4];
+    ldmatrix_x4_trans(b, b0 + (kb * 16 + (mat & 1) * 8 + mr) * pitch + (mat >> 1) * 8);
+#pragma unroll
+    for (int rb = kb; rb < 4; ++rb) {
+      const uint4 x = xf[lower_block(rb, kb) * 32 + lane];
+      const uint32_t a[4] = {x.x, x.y, x.z, x.w};
+      mma_bf16(acc[rb][0], a, b[0], b[1]);
+      mma_bf16(acc[rb][1], a, b[2], b[3]);
+    }
   }
 }
 
@@ -94,450 +163,460 @@ __device__ __forceinline__ void load_rows(__nv_bfloat16* dst, int ld, const __nv
 // ------------------------------------------------------------------------------------------------------------------
 struct PrepSmem {
   __nv_bfloat16 k[kC][kLdK];
-  __nv_bfloat16 kb[kC][kLdK];     // beta k, later beta k exp(gc)
-  float L[kC][kLdF];              // strictly lower part of the system, later staging of output tiles
-  float A[kC][kLdF];              // (I + L)^-1
-  __nv_bfloat16 Ab[kC][kLdC];
+  union {
+    float A[kC * kFp];                 // L, then (I + L)^-1
+    struct {
+      uint4 uf[kBlocks * 32];          // fragments of A beta
+      uint4 wf[kBlocks * 32];          // fragments of A beta exp(gc)
+    };
+  };
   float gc[kC];
   float beta[kC];
-  // followed by vb [64][V + 8] bf16
+  // followed by v [64][V + 8] bf16
 };
 
-__global__ void __launch_bounds__(kThreads) gdn_chunk_prepare(const ChunkParams p) {
+__global__ void __launch_bounds__(kThreads, 3) gdn_chunk_prepare(const ChunkParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   PrepSmem& s = *reinterpret_cast<PrepSmem*>(smem_raw);
-  __nv_bfloat16* vb = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(PrepSmem));
+  __nv_bfloat16* vs = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(PrepSmem));
   const int ldv = p.V + 8;
   const int c = blockIdx.x, h = blockIdx.y;
-  const int64_t t0 = p.chunk_t0[c];
-  const int n = chunk_len(p, c);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-  load_rows(&s.k[0][0], kLdK, p.k, t0, n, p.H, h, kK, 0, kK);
-  load_rows(vb, ldv, p.v, t0, n, p.H, h, p.V, 0, p.V);
-  if (threadIdx.x < kC) {
-    const int r = threadIdx.x;
-    s.beta[r] = r < n ? __bfloat162float(p.beta[(t0 + r) * p.H + h]) : 0.f;
-    s.gc[r] = r < n ? p.g[(t0 + r) * p.H + h] : 0.f;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    // inclusive scan of 64 values by one warp: two per lane
-    float a = s.gc[2 * lane], b = s.gc[2 * lane + 1];
-    float sum = a + b, pre = sum;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mat = lane >> 3, mr = lane & 7;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (c >= p.seq_chunk0[p.N]) return;
+  const ChunkPos cp = chunk_pos(p, c);
+  const int64_t Hk = static_cast<int64_t>(p.H) * kK, Hv = static_cast<int64_t>(p.H) * p.V;
+  load_tile(&s.k[0][0], kLdK, p.k + cp.t0 * Hk + h * kK, Hk, kK, cp.n, kThreads);
+  cp_async_commit();
+  load_tile(vs, ldv, p.v + cp.t0 * Hv + static_cast<int64_t>(h) * p.V, Hv, p.V, cp.n, kThreads);
+  cp_async_commit();
+  const int64_t ch = static_cast<int64_t>(c) * p.H + h;
+  if (warp == 0) {                      // inclusive scan of the log decays, two tokens per lane
+    const int t = 2 * lane;
+    const float a = t < cp.n ? p.g[(cp.t0 + t) * p.H + h] : 0.f;
+    const float b = t + 1 < cp.n ? p.g[(cp.t0 + t + 1) * p.H + h] : 0.f;
+    const float sum = a + b;
+    float pre = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, pre, o);
-      if (lane >= o) pre += t;
+      const float x = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += x;
     }
     const float base = pre - sum;
-    s.gc[2 * lane] = base + a;
-    s.gc[2 * lane + 1] = base + a + b;
+    s.gc[t] = base + a;
+    s.gc[t + 1] = base + a + b;
+    if (t < cp.n) p.gcum[(cp.t0 + t) * p.H + h] = base + a;
+    if (t + 1 < cp.n) p.gcum[(cp.t0 + t + 1) * p.H + h] = base + a + b;
+    if (lane == 31) p.decay[ch] = __expf(base + a + b);
+  } else if (warp == 1) {
+    s.beta[lane] = lane < cp.n ? __bfloat162float(p.beta[(cp.t0 + lane) * p.H + h]) : 0.f;
+    s.beta[lane + 32] = lane + 32 < cp.n ? __bfloat162float(p.beta[(cp.t0 + lane + 32) * p.H + h]) : 0.f;
   }
+  cp_async_wait<1>();
   __syncthreads();
-  if (threadIdx.x < n) p.gcum[(t0 + threadIdx.x) * p.H + h] = s.gc[threadIdx.x];
-  // kb = beta k, vb = beta v
-  for (int i = threadIdx.x; i < kC * (kK / 2); i += kThreads) {
-    const int r = i / (kK / 2), cc = (i - r * (kK / 2)) * 2;
-    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&s.k[r][cc]));
-    *reinterpret_cast<__nv_bfloat162*>(&s.kb[r][cc]) = __floats2bfloat162_rn(f.x * s.beta[r], f.y * s.beta[r]);
+  for (int i = warp; i < kBlocks; i += kThreads / 32) {
+    const int bi = block_row(i), bj = i - lower_block(bi, 0);
+    float acc[2][4];
+    score_block(&s.k[0][0], &s.k[0][0], bi, bj, acc);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = bi * 16 + g + 8 * (e >> 1), cc = bj * 16 + j * 8 + 2 * t4 + (e & 1);
+        s.A[r * kFp + cc] = r > cc ? acc[j][e] * s.beta[r] * __expf(s.gc[r] - s.gc[cc]) : 0.f;
+      }
   }
-  for (int i = threadIdx.x; i < kC * (p.V / 2); i += kThreads) {
-    const int r = i / (p.V / 2), cc = (i - r * (p.V / 2)) * 2;
-    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vb + r * ldv + cc));
-    *reinterpret_cast<__nv_bfloat162*>(vb + r * ldv + cc) = __floats2bfloat162_rn(f.x * s.beta[r], f.y * s.beta[r]);
-  }
-  __syncthreads();
-  // L = (beta k) k^T: warp w owns rows [16 w, 16 w + 16)
+  // kd^T as A fragments, a warp per 16 rows of K
   {
-    FragC acc[4];
+    const float gl = s.gc[kC - 1];
+    uint4* dst = p.kd + ch * kWFrag + warp * 4 * 32 + lane;
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::fill_fragment(acc[nt], 0.f);
-    for (int ks = 0; ks < kK / 16; ++ks) {
-      FragA a;
-      wmma::load_matrix_sync(a, &s.kb[16 * warp][16 * ks], kLdK);
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t a[4];
+      ldmatrix_x4_trans(a, &s.k[ks * 16 + (mat >> 1) * 8 + mr][warp * 16 + (mat & 1) * 8]);
+      const int t = ks * 16 + 2 * t4;
+      const float f[4] = {__expf(gl - s.gc[t]), __expf(gl - s.gc[t + 1]), __expf(gl - s.gc[t + 8]), __expf(gl - s.gc[t + 9])};
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        FragBT b;   // B[kk][nn] = k[16 nt + nn][16 ks + kk]
-        wmma::load_matrix_sync(b, &s.k[16 * nt][16 * ks], kLdK);
-        wmma::mma_sync(acc[nt], a, b, acc[nt]);
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack_bf16x2(a[e]);
+        a[e] = pack_bf16x2(x.x * f[2 * (e >> 1)], x.y * f[2 * (e >> 1) + 1]);
       }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.L[16 * warp][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kC * kC; i += kThreads) {
-    const int r = i / kC, cc = i - r * kC;
-    s.L[r][cc] = (r > cc) ? s.L[r][cc] * __expf(s.gc[r] - s.gc[cc]) : 0.f;
-  }
-  __syncthreads();
-  // (I + L) A = I by forward substitution; thread j < 64 owns column j of A (its first j rows are zero)
-  if (threadIdx.x < kC) {
-    const int j = threadIdx.x;
-    for (int i = 0; i < kC; ++i) {
-      float acc = (i == j) ? 1.f : 0.f;
-      for (int m = j; m < i; ++m) acc -= s.L[i][m] * s.A[m][j];
-      s.A[i][j] = (i >= j) ? acc : 0.f;
+      dst[ks * 32] = make_uint4(a[0], a[1], a[2], a[3]);
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kC * kC; i += kThreads) {
-    const int r = i / kC, cc = i - r * kC;
-    s.Ab[r][cc] = __float2bfloat16(s.A[r][cc]);
-    if (p.a_out != nullptr && r < n) p.a_out[((t0 + r) * p.H + h) * kC + cc] = s.A[r][cc];
-  }
-  // kb <- beta k exp(gc)
-  for (int i = threadIdx.x; i < kC * (kK / 2); i += kThreads) {
-    const int r = i / (kK / 2), cc = (i - r * (kK / 2)) * 2;
-    const float e = __expf(s.gc[r]);
-    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&s.kb[r][cc]));
-    *reinterpret_cast<__nv_bfloat162*>(&s.kb[r][cc]) = __floats2bfloat162_rn(f.x * e, f.y * e);
-  }
-  __syncthreads();
-  // w = A kb  [64 x 128],  u = A vb  [64 x V]; 64 output columns at a time through the warp's rows of L (staging)
-  __nv_bfloat16* wout = p.w + (static_cast<int64_t>(c) * p.H + h) * kC * kK;
-  __nv_bfloat16* uout = p.u + (static_cast<int64_t>(c) * p.H + h) * kC * p.V;
-  const int passes_w = kK / 64, passes_u = p.V / 64;
-  for (int ps = 0; ps < passes_w + passes_u; ++ps) {
-    const bool is_w = ps < passes_w;
-    const int col0 = (is_w ? ps : ps - passes_w) * 64;
-    const __nv_bfloat16* bsrc = is_w ? &s.kb[0][0] : vb;
-    const int ldb = is_w ? kLdK : ldv;
-    FragC acc[4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::fill_fragment(acc[nt], 0.f);
-    for (int ks = 0; ks < kC / 16; ++ks) {
-      FragA a;
-      wmma::load_matrix_sync(a, &s.Ab[16 * warp][16 * ks], kLdC);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        FragB b;
-        wmma::load_matrix_sync(b, bsrc + (16 * ks) * ldb + col0 + 16 * nt, ldb);
-        wmma::mma_sync(acc[nt], a, b, acc[nt]);
-      }
+  invert_unit_lower<kThreads>(s.A);
+  if (p.a_out != nullptr) {
+    for (int i = threadIdx.x; i < kC * kC; i += kThreads) {
+      const int r = i / kC, cc = i - r * kC;
+      if (r < cp.n) p.a_out[((cp.t0 + r) * p.H + h) * kC + cc] = r >= cc ? s.A[r * kFp + cc] : 0.f;
     }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.L[16 * warp][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
-    __syncwarp();
-    __nv_bfloat16* dst = is_w ? wout : uout;
-    const int ldo = is_w ? kK : p.V;
-    for (int i = lane; i < 16 * 32; i += 32) {
-      const int r = 16 * warp + i / 32, cc = (i % 32) * 2;
-      *reinterpret_cast<__nv_bfloat162*>(dst + r * ldo + col0 + cc) = __floats2bfloat162_rn(s.L[r][cc], s.L[r][cc + 1]);
-    }
-    __syncwarp();
   }
-}
-
-// ------------------------------------------------------------------------------------------------------------------
-// Kernel 2: per (V tile, head, sequence), sequential over the chunks.  The pass is a chain of small dependent steps, so
-// everything a chunk needs from global memory (w, its u slice, k, the cumulative decay) is fetched one chunk ahead with
-// cp.async into a second shared-memory stage while the current chunk is computed.
-// ------------------------------------------------------------------------------------------------------------------
-struct StateStage {
-  __nv_bfloat16 w[kC][kLdK];
-  __nv_bfloat16 k[kC][kLdK];        // k, turned into k exp(gc_last - gc) in place
-  __nv_bfloat16 u[kC][kLdC];
-  float gc[kC];
-};
-struct StateSmem {
-  float S[kK][kLdF];                // state columns [v0, v0 + 64)
-  __nv_bfloat16 Sb[kK][kLdC];       // bf16 copy for the tensor cores
-  float vf[kC][kLdF];               // w S
-  __nv_bfloat16 vn[kC][kLdC];       // v_new
-  StateStage st[2];
-};
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ void state_prefetch(const ChunkParams& p, StateStage& st, int c, int h, int v0) {
-  const int64_t t0 = p.chunk_t0[c];
-  const int n = chunk_len(p, c);
-  const int64_t ch = static_cast<int64_t>(c) * p.H + h;
-  const __nv_bfloat16* wsrc = p.w + ch * kC * kK;
-  for (int i = threadIdx.x; i < kC * (kK / 8); i += kThreads) {
-    const int r = i / (kK / 8), cc = (i - r * (kK / 8)) * 8;
-    cp_async16(&st.w[r][cc], wsrc + r * kK + cc);
-    if (r < n) cp_async16(&st.k[r][cc], p.k + ((t0 + r) * p.H + h) * kK + cc);
-    else *reinterpret_cast<uint4*>(&st.k[r][cc]) = make_uint4(0u, 0u, 0u, 0u);
-  }
-  const __nv_bfloat16* usrc = p.u + ch * kC * p.V + v0;
-  for (int i = threadIdx.x; i < kC * (kVT / 8); i += kThreads) {
-    const int r = i / (kVT / 8), cc = (i - r * (kVT / 8)) * 8;
-    cp_async16(&st.u[r][cc], usrc + static_cast<int64_t>(r) * p.V + cc);
-  }
-  if (threadIdx.x < kC) {
-    const int r = min(static_cast<int>(threadIdx.x), n - 1);    // padded rows keep the last value (their g is 0)
-    cp_async4(&st.gc[threadIdx.x], p.gcum + (t0 + r) * p.H + h);
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) gdn_chunk_state(const ChunkParams p) {
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  StateSmem& s = *reinterpret_cast<StateSmem*>(smem_raw);
-  const int vt = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
-  const int v0 = vt * kVT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t st_off = (static_cast<int64_t>(seq) * p.H + h) * kK * p.V;
-  const int c_begin = p.seq_chunk0[seq], c_end = p.seq_chunk0[seq + 1];
-  if (c_begin < c_end) state_prefetch(p, s.st[0], c_begin, h, v0);
-  cp_async_commit();
-  for (int i = threadIdx.x; i < kK * kVT; i += kThreads) {
-    const int r = i / kVT, cc = i - r * kVT;
-    const float val = p.h0 ? p.h0[st_off + static_cast<int64_t>(r) * p.V + v0 + cc] : 0.f;
-    s.S[r][cc] = val;
-    s.Sb[r][cc] = __float2bfloat16(val);
-  }
-  for (int c = c_begin; c < c_end; ++c) {
-    StateStage& cur = s.st[(c - c_begin) & 1];
-    // the other stage was last read two barriers ago (end of the previous iteration)
-    if (c + 1 < c_end) state_prefetch(p, s.st[(c - c_begin + 1) & 1], c + 1, h, v0);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();   // stage `cur` (and, in the first iteration, S / Sb) visible to every warp
-    const int64_t ch = static_cast<int64_t>(c) * p.H + h;
-    // chunk-start state for the output kernel
-    {
-      __nv_bfloat16* hdst = p.hstate + ch * kK * p.V + v0;
-      for (int i = threadIdx.x; i < kK * (kVT / 8); i += kThreads) {
-        const int r = i / (kVT / 8), cc = (i - r * (kVT / 8)) * 8;
-        *reinterpret_cast<uint4*>(hdst + static_cast<int64_t>(r) * p.V + cc) = *reinterpret_cast<const uint4*>(&s.Sb[r][cc]);
-      }
+  // the fragments of A beta and A beta exp(gc) take the place of A
+  {
+    uint4 fu[2], fw[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = warp + 8 * r;
+      if (i >= kBlocks) break;
+      const int bi = block_row(i), c0 = (i - lower_block(bi, 0)) * 16 + 2 * t4;
+      const float* a = s.A + (bi * 16 + g) * kFp + c0;
+      const float* b = a + 8 * kFp;
+      const float b0 = s.beta[c0], b1 = s.beta[c0 + 1], b2 = s.beta[c0 + 8], b3 = s.beta[c0 + 9];
+      const float x[4] = {a[0] * b0, a[1] * b1, b[0] * b0, b[1] * b1}, y[4] = {a[8] * b2, a[9] * b3, b[8] * b2, b[9] * b3};
+      const float e0 = __expf(s.gc[c0]), e1 = __expf(s.gc[c0 + 1]), e2 = __expf(s.gc[c0 + 8]), e3 = __expf(s.gc[c0 + 9]);
+      const float xe[4] = {x[0] * e0, x[1] * e1, x[2] * e0, x[3] * e1}, ye[4] = {y[0] * e2, y[1] * e3, y[2] * e2, y[3] * e3};
+      fu[r] = pack_tiles(x, y);
+      fw[r] = pack_tiles(xe, ye);
     }
-    // vf = w S   (rows of this warp)
-    {
-      FragC acc[4];
+    __syncthreads();
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) wmma::fill_fragment(acc[nt], 0.f);
-#pragma unroll
-      for (int ks = 0; ks < kK / 16; ++ks) {
-        FragA a;
-        wmma::load_matrix_sync(a, &cur.w[16 * warp][16 * ks], kLdK);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          FragB b;
-          wmma::load_matrix_sync(b, &s.Sb[16 * ks][16 * nt], kLdC);
-          wmma::mma_sync(acc[nt], a, b, acc[nt]);
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.vf[16 * warp][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
+    for (int r = 0; r < 2; ++r) {
+      const int i = warp + 8 * r;
+      if (i >= kBlocks) break;
+      s.uf[i * 32 + lane] = fu[r];
+      s.wf[i * 32 + lane] = fw[r];
     }
-    __syncwarp();
-    const float g_last = cur.gc[kC - 1];
-    // v_new = u - w S for the warp's own 16 rows (bf16, to shared and global); k <- k exp(g_last - gc) for the same rows
-    {
-      __nv_bfloat16* vdst = p.vnew + ch * kC * p.V + v0;
-      for (int i = lane; i < 16 * (kVT / 2); i += 32) {
-        const int r = 16 * warp + i / (kVT / 2), cc = (i % (kVT / 2)) * 2;
-        const float2 uu = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&cur.u[r][cc]));
-        const __nv_bfloat162 o = __floats2bfloat162_rn(uu.x - s.vf[r][cc], uu.y - s.vf[r][cc + 1]);
-        *reinterpret_cast<__nv_bfloat162*>(&s.vn[r][cc]) = o;
-        *reinterpret_cast<__nv_bfloat162*>(vdst + static_cast<int64_t>(r) * p.V + cc) = o;
-      }
-      for (int i = lane; i < 16 * (kK / 2); i += 32) {
-        const int r = 16 * warp + i / (kK / 2), cc = (i % (kK / 2)) * 2;
-        const float e = __expf(g_last - cur.gc[r]);
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&cur.k[r][cc]));
-        *reinterpret_cast<__nv_bfloat162*>(&cur.k[r][cc]) = __floats2bfloat162_rn(f.x * e, f.y * e);
-      }
-    }
-    __syncthreads();   // vn and the scaled k of all rows are complete; every warp is done reading Sb
-    // S <- S exp(g_last) + kd^T v_new: warp w owns state rows [32 w, 32 w + 32)
-    {
-      const float dec = __expf(g_last);
-#pragma unroll
-      for (int rt = 0; rt < 2; ++rt) {
-        const int row0 = 32 * warp + 16 * rt;
-        FragC acc[4];
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          wmma::load_matrix_sync(acc[nt], &s.S[row0][16 * nt], kLdF, wmma::mem_row_major);
-#pragma unroll
-          for (int e = 0; e < acc[nt].num_elements; ++e) acc[nt].x[e] *= dec;
-        }
-#pragma unroll
-        for (int ks = 0; ks < kC / 16; ++ks) {
-          FragAT a;   // A[m][kk] = kd[16 ks + kk][row0 + m]
-          wmma::load_matrix_sync(a, &cur.k[16 * ks][row0], kLdK);
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt) {
-            FragB b;
-            wmma::load_matrix_sync(b, &s.vn[16 * ks][16 * nt], kLdC);
-            wmma::mma_sync(acc[nt], a, b, acc[nt]);
-          }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.S[row0][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
-      }
-      __syncwarp();
-      for (int i = lane; i < 32 * (kVT / 2); i += 32) {
-        const int r = 32 * warp + i / (kVT / 2), cc = (i % (kVT / 2)) * 2;
-        *reinterpret_cast<__nv_bfloat162*>(&s.Sb[r][cc]) = __floats2bfloat162_rn(s.S[r][cc], s.S[r][cc + 1]);
-      }
-    }
-    __syncthreads();   // the new Sb is complete; stage `cur` may be overwritten by the prefetch of the next iteration
   }
   cp_async_wait<0>();
   __syncthreads();
-  if (p.ht != nullptr) {
-    for (int i = threadIdx.x; i < kK * kVT; i += kThreads) {
-      const int r = i / kVT, cc = i - r * kVT;
-      p.ht[st_off + static_cast<int64_t>(r) * p.V + v0 + cc] = s.S[r][cc];
-    }
+  // w: a warp per 16 columns of K; u: a warp per 16 columns of V
+  {
+    float acc[4][2][4];
+    lower_times(acc, s.wf, &s.k[0][warp * 16], kLdK);
+    uint4* dst = p.w + ch * kWFrag + warp * 32 + lane;
+#pragma unroll
+    for (int rb = 0; rb < 4; ++rb) dst[rb * kKs * 32] = pack_tiles(acc[rb][0], acc[rb][1]);
+  }
+  const int vt = p.V / 16;
+  for (int t = warp; t < vt; t += kThreads / 32) {
+    float acc[4][2][4];
+    lower_times(acc, s.uf, vs + t * 16, ldv);
+    uint4* dst = p.u + (ch * vt + t) * kUFrag + lane;
+#pragma unroll
+    for (int rb = 0; rb < 4; ++rb) dst[rb * 32] = pack_tiles(acc[rb][0], acc[rb][1]);
   }
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Kernel 3: per (chunk, head, V tile)
+// Kernel 2: per (16 NP columns of V, head, sequence), sequential over the chunks.  Four warps: in the first product a warp owns 16
+// tokens, in the second 32 rows of the state, which stays in its registers in fp32.  A chunk is two dependent products with an
+// exchange through shared memory after each (S and v_new as B operands), about 500 cycles; its operands (34 KB) arrive STAGES - 1
+// chunks ahead through cp.async.  The 16 columns keep the serial part short and spread 16 heads over 128 SMs; two such CTAs
+// share an SM when there are more, and beyond two per SM a CTA takes 32 columns, which halves the operand traffic.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int kStateThreads = 128;
+template <int NP>
+struct StateLay {
+  static constexpr int kStage = (2 * kWFrag + NP * kUFrag);      // uint4 of a stage: w | kd | u
+  static constexpr int kPitch = NP * 16 + 8;                     // bf16 pitch of the exchange buffers
+  static constexpr int smem(int stages) { return stages * kStage * 16 + (kK + kC) * kPitch * 2; }
+};
+
+template <int NP, int STAGES>
+__global__ void __launch_bounds__(kStateThreads, 1) gdn_chunk_state(const ChunkParams p) {
+  using L = StateLay<NP>;
+  constexpr int kPitch = L::kPitch;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  uint4* ring = reinterpret_cast<uint4*>(smem_raw);
+  __nv_bfloat16* sb = reinterpret_cast<__nv_bfloat16*>(ring + STAGES * L::kStage);     // [128][pitch] S
+  __nv_bfloat16* vb = sb + kK * kPitch;                                                // [64][pitch] v_new
+  const int tile0 = blockIdx.x * NP, h = blockIdx.y, seq = blockIdx.z, vt = p.V / 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mat = lane >> 3, mr = lane & 7;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int c0 = p.seq_chunk0[seq], nc = p.seq_chunk0[seq + 1] - c0;
+  const int64_t st_off = ((static_cast<int64_t>(seq) * p.H + h) * kK + warp * 32 + g) * p.V + tile0 * 16 + 2 * t4;
+  float S[2][2 * NP][4];
+#pragma unroll
+  for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+    for (int j = 0; j < 2 * NP; ++j) {
+      zero(S[rb][j]);
+      if (p.h0 != nullptr) {
+        const float* src = p.h0 + st_off + static_cast<int64_t>(rb * 16) * p.V + j * 8;
+        const float2 a = *reinterpret_cast<const float2*>(src), b = *reinterpret_cast<const float2*>(src + 8 * p.V);
+        S[rb][j][0] = a.x; S[rb][j][1] = a.y; S[rb][j][2] = b.x; S[rb][j][3] = b.y;
+      }
+    }
+  auto fetch = [&](int i) {            // chunk i of the sequence into stage i % STAGES
+    if (i < nc) {
+      const int64_t ch = static_cast<int64_t>(c0 + i) * p.H + h;
+      uint4* st = ring + (i % STAGES) * L::kStage;
+      const uint4 *w = p.w + ch * kWFrag, *kd = p.kd + ch * kWFrag, *u = p.u + (ch * vt + tile0) * kUFrag;
+#pragma unroll
+      for (int e = 0; e < kWFrag / kStateThreads; ++e) {
+        const int at = e * kStateThreads + threadIdx.x;
+        cp_async16(st + at, w + at, true);
+        cp_async16(st + kWFrag + at, kd + at, true);
+      }
+#pragma unroll
+      for (int e = 0; e < NP; ++e) {
+        const int at = e * kStateThreads + threadIdx.x;
+        cp_async16(st + 2 * kWFrag + at, u + at, true);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < STAGES - 1; ++i) fetch(i);
+  float dec_next = nc > 0 ? p.decay[static_cast<int64_t>(c0) * p.H + h] : 0.f;
+  cp_async_wait<STAGES - 2>();
+  __syncthreads();
+  uint4 wf[kKs];                       // this warp's 16 rows of w, loaded one chunk ahead
+#pragma unroll
+  for (int ks = 0; ks < kKs; ++ks) wf[ks] = ring[(warp * kKs + ks) * 32 + lane];
+  for (int i = 0; i < nc; ++i) {
+    const int64_t ch = static_cast<int64_t>(c0 + i) * p.H + h;
+    const uint4* st = ring + (i % STAGES) * L::kStage;
+    const float dec = dec_next;
+    // S as bf16 for the tensor cores
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int j = 0; j < 2 * NP; ++j) {
+        __nv_bfloat16* dst = sb + (warp * 32 + rb * 16 + g) * kPitch + j * 8 + 2 * t4;
+        *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(S[rb][j][0], S[rb][j][1]);
+        *reinterpret_cast<uint32_t*>(dst + 8 * kPitch) = pack_bf16x2(S[rb][j][2], S[rb][j][3]);
+      }
+    __syncthreads();                   // S complete; every warp has left the previous chunk, so its stage and v_new are free
+    fetch(i + STAGES - 1);
+    if (i + 1 < nc) dec_next = p.decay[ch + p.H];
+    uint4 kf[2][4], uf[NP];
+#pragma unroll
+    for (int t = 0; t < NP; ++t) uf[t] = st[2 * kWFrag + t * kUFrag + warp * 32 + lane];
+    // w S: even and odd k-steps in sums of their own, so that the chain of dependent products is half as long
+    float acc[2][2 * NP][4];
+#pragma unroll
+    for (int j = 0; j < 2 * NP; ++j) {
+      zero(acc[0][j]);
+      zero(acc[1][j]);
+    }
+#pragma unroll
+    for (int ks = 0; ks < kKs; ++ks) {
+      const uint32_t a[4] = {wf[ks].x, wf[ks].y, wf[ks].z, wf[ks].w};
+#pragma unroll
+      for (int t = 0; t < NP; ++t) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, sb + (ks * 16 + (mat & 1) * 8 + mr) * kPitch + t * 16 + (mat >> 1) * 8);
+        mma_bf16(acc[ks & 1][2 * t], a, b[0], b[1]);
+        mma_bf16(acc[ks & 1][2 * t + 1], a, b[2], b[3]);
+        if ((ks >> 1) == warp)         // the state before this chunk, for the output kernel
+          p.hstate[((ch * vt + tile0 + t) * kKs + ks) * 32 + lane] = make_uint4(b[0], b[1], b[2], b[3]);
+      }
+    }
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) kf[rb][ks] = st[kWFrag + ((warp * 2 + rb) * 4 + ks) * 32 + lane];
+    // v_new = u - w S
+#pragma unroll
+    for (int t = 0; t < NP; ++t) {
+      const uint32_t uw[4] = {uf[t].x, uf[t].y, uf[t].z, uf[t].w};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 a = unpack_bf16x2(uw[2 * j]), b = unpack_bf16x2(uw[2 * j + 1]);
+        __nv_bfloat16* dst = vb + (warp * 16 + g) * kPitch + t * 16 + j * 8 + 2 * t4;
+        const float (&x)[4] = acc[0][2 * t + j], (&y)[4] = acc[1][2 * t + j];
+        *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(a.x - (x[0] + y[0]), a.y - (x[1] + y[1]));
+        *reinterpret_cast<uint32_t*>(dst + 8 * kPitch) = pack_bf16x2(b.x - (x[2] + y[2]), b.y - (x[3] + y[3]));
+      }
+    }
+    cp_async_wait<STAGES - 2>();       // the next chunk's operands (this thread's part)
+    __syncthreads();                   // v_new and the next stage complete
+    {
+      const uint4* nx = ring + ((i + 1) % STAGES) * L::kStage;
+#pragma unroll
+      for (int ks = 0; ks < kKs; ++ks) wf[ks] = nx[(warp * kKs + ks) * 32 + lane];
+    }
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int j = 0; j < 2 * NP; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[rb][j][e] *= dec;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int t = 0; t < NP; ++t) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, vb + (ks * 16 + (mat & 1) * 8 + mr) * kPitch + t * 16 + (mat >> 1) * 8);
+#pragma unroll
+        for (int rb = 0; rb < 2; ++rb) {
+          const uint32_t a[4] = {kf[rb][ks].x, kf[rb][ks].y, kf[rb][ks].z, kf[rb][ks].w};
+          mma_bf16(S[rb][2 * t], a, b[0], b[1]);
+          mma_bf16(S[rb][2 * t + 1], a, b[2], b[3]);
+        }
+        if (ks == warp) p.vnew[((ch * vt + tile0 + t) * 4 + ks) * 32 + lane] = make_uint4(b[0], b[1], b[2], b[3]);
+      }
+  }
+  cp_async_wait<0>();
+  if (p.ht != nullptr) {
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int j = 0; j < 2 * NP; ++j) {
+        float* dst = p.ht + st_off + static_cast<int64_t>(rb * 16) * p.V + j * 8;
+        *reinterpret_cast<float2*>(dst) = make_float2(S[rb][j][0], S[rb][j][1]);
+        *reinterpret_cast<float2*>(dst + 8 * p.V) = make_float2(S[rb][j][2], S[rb][j][3]);
+      }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// Kernel 3: per (chunk, head).  A warp owns 16 columns of V for RB of the four row blocks, so that S and v_new go from memory to
+// its registers once; q and the masked scores are the shared operands.
 // ------------------------------------------------------------------------------------------------------------------
 struct OutSmem {
   __nv_bfloat16 q[kC][kLdK];
   __nv_bfloat16 k[kC][kLdK];
-  float P[kC][kLdF];               // q k^T, later staging of the output tile
-  __nv_bfloat16 Pb[kC][kLdC];
+  uint4 pf[kBlocks * 32];          // masked, decayed scores as A fragments
   float gc[kC];
 };
 
-__global__ void __launch_bounds__(kThreads) gdn_chunk_output(const ChunkParams p) {
+template <int RB>
+__global__ void __launch_bounds__(kThreads, 2) gdn_chunk_output(const ChunkParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   OutSmem& s = *reinterpret_cast<OutSmem*>(smem_raw);
-  const int c = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kVT;
-  const int64_t t0 = p.chunk_t0[c];
-  const int n = chunk_len(p, c);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ch = static_cast<int64_t>(c) * p.H + h;
-  load_rows(&s.q[0][0], kLdK, p.q, t0, n, p.H, h, kK, 0, kK);
-  load_rows(&s.k[0][0], kLdK, p.k, t0, n, p.H, h, kK, 0, kK);
-  if (threadIdx.x < kC) {
-    const int r = min(static_cast<int>(threadIdx.x), n - 1);
-    s.gc[threadIdx.x] = p.gcum[(t0 + r) * p.H + h];
+  const int c = blockIdx.x, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mat = lane >> 3, mr = lane & 7;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (c >= p.seq_chunk0[p.N]) return;
+  const ChunkPos cp = chunk_pos(p, c);
+  const int64_t Hk = static_cast<int64_t>(p.H) * kK, ch = static_cast<int64_t>(c) * p.H + h;
+  load_tile(&s.q[0][0], kLdK, p.q + cp.t0 * Hk + h * kK, Hk, kK, cp.n, kThreads);
+  load_tile(&s.k[0][0], kLdK, p.k + cp.t0 * Hk + h * kK, Hk, kK, cp.n, kThreads);
+  cp_async_commit();
+  constexpr int kParts = 4 / RB, kTiles = kThreads / 32 / kParts;      // warps side by side
+  const int part = warp / kTiles, vt = p.V / 16;
+  uint4 sf[kKs], vf[4];
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int ks = 0; ks < kKs; ++ks) sf[ks] = p.hstate[((ch * vt + t) * kKs + ks) * 32 + lane];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) vf[ks] = p.vnew[((ch * vt + t) * 4 + ks) * 32 + lane];
+  };
+  const int t_first = warp % kTiles;
+  if (t_first < vt) fetch(t_first);
+  if (threadIdx.x < kC) s.gc[threadIdx.x] = p.gcum[(cp.t0 + min(static_cast<int>(threadIdx.x), cp.n - 1)) * p.H + h];
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int i = warp; i < kBlocks; i += kThreads / 32) {
+    const int bi = block_row(i), bj = i - lower_block(bi, 0);
+    float acc[2][4];
+    score_block(&s.q[0][0], &s.k[0][0], bi, bj, acc);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = bi * 16 + g + 8 * (e >> 1), cc = bj * 16 + j * 8 + 2 * t4 + (e & 1);
+        acc[j][e] = r >= cc ? acc[j][e] * __expf(s.gc[r] - s.gc[cc]) : 0.f;
+      }
+    s.pf[i * 32 + lane] = pack_tiles(acc[0], acc[1]);
   }
   __syncthreads();
-  {
-    FragC acc[4];
+  for (int t = t_first; t < vt; t += kTiles) {
+    if (t != t_first) fetch(t);
+    float acc[RB][2][4];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::fill_fragment(acc[nt], 0.f);
-    for (int ks = 0; ks < kK / 16; ++ks) {
-      FragA a;
-      wmma::load_matrix_sync(a, &s.q[16 * warp][16 * ks], kLdK);
+    for (int r = 0; r < RB; ++r) {
+      const int rb = part * RB + r;
+      zero(acc[r][0]);
+      zero(acc[r][1]);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        FragBT b;
-        wmma::load_matrix_sync(b, &s.k[16 * nt][16 * ks], kLdK);
-        wmma::mma_sync(acc[nt], a, b, acc[nt]);
+      for (int ks = 0; ks < kKs; ++ks) {
+        uint32_t a[4];
+        ldmatrix_x4(a, &s.q[rb * 16 + (mat & 1) * 8 + mr][ks * 16 + (mat >> 1) * 8]);
+        mma_bf16(acc[r][0], a, sf[ks].x, sf[ks].y);
+        mma_bf16(acc[r][1], a, sf[ks].z, sf[ks].w);
+      }
+      const float e0 = __expf(s.gc[rb * 16 + g]), e1 = __expf(s.gc[rb * 16 + g + 8]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        acc[r][j][0] *= e0; acc[r][j][1] *= e0;
+        acc[r][j][2] *= e1; acc[r][j][3] *= e1;
+      }
+#pragma unroll
+      for (int kb = 0; kb < 4; ++kb) {
+        if (kb > rb) break;
+        const uint4 x = s.pf[lower_block(rb, kb) * 32 + lane];
+        const uint32_t a[4] = {x.x, x.y, x.z, x.w};
+        mma_bf16(acc[r][0], a, vf[kb].x, vf[kb].y);
+        mma_bf16(acc[r][1], a, vf[kb].z, vf[kb].w);
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int row = rb * 16 + g + 8 * half;
+        if (row >= cp.n) continue;
+        __nv_bfloat16* dst = p.o + ((cp.t0 + row) * p.H + h) * p.V + t * 16 + 2 * t4;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          *reinterpret_cast<uint32_t*>(dst + j * 8) = pack_bf16x2(acc[r][j][2 * half] * p.scale, acc[r][j][2 * half + 1] * p.scale);
       }
     }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.P[16 * warp][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
   }
-  __syncthreads();   // every warp is done with q as it was loaded
-  for (int i = threadIdx.x; i < kC * kC; i += kThreads) {
-    const int r = i / kC, cc = i - r * kC;
-    s.Pb[r][cc] = __float2bfloat16(r >= cc ? s.P[r][cc] * __expf(s.gc[r] - s.gc[cc]) : 0.f);
-  }
-  for (int i = threadIdx.x; i < kC * (kK / 2); i += kThreads) {
-    const int r = i / (kK / 2), cc = (i - r * (kK / 2)) * 2;
-    const float e = __expf(s.gc[r]);
-    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&s.q[r][cc]));
-    *reinterpret_cast<__nv_bfloat162*>(&s.q[r][cc]) = __floats2bfloat162_rn(f.x * e, f.y * e);
-  }
-  __syncthreads();
-  {
-    const __nv_bfloat16* hsrc = p.hstate + ch * kK * p.V + v0;
-    const __nv_bfloat16* vsrc = p.vnew + ch * kC * p.V + v0;
-    FragC acc[4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::fill_fragment(acc[nt], 0.f);
-    for (int ks = 0; ks < kK / 16; ++ks) {
-      FragA a;
-      wmma::load_matrix_sync(a, &s.q[16 * warp][16 * ks], kLdK);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        FragB b;
-        wmma::load_matrix_sync(b, hsrc + static_cast<int64_t>(16 * ks) * p.V + 16 * nt, p.V);
-        wmma::mma_sync(acc[nt], a, b, acc[nt]);
-      }
-    }
-    for (int ks = 0; ks < kC / 16; ++ks) {
-      FragA a;
-      wmma::load_matrix_sync(a, &s.Pb[16 * warp][16 * ks], kLdC);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        FragB b;
-        wmma::load_matrix_sync(b, vsrc + static_cast<int64_t>(16 * ks) * p.V + 16 * nt, p.V);
-        wmma::mma_sync(acc[nt], a, b, acc[nt]);
-      }
-    }
-    // P rows of this warp were last read (as P) before the barrier above: reuse them as staging
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) wmma::store_matrix_sync(&s.P[16 * warp][16 * nt], acc[nt], kLdF, wmma::mem_row_major);
-  }
-  __syncwarp();
-  for (int i = lane; i < 16 * (kVT / 2); i += 32) {
-    const int r = 16 * warp + i / (kVT / 2), cc = (i % (kVT / 2)) * 2;
-    if (r < n)
-      *reinterpret_cast<__nv_bfloat162*>(p.o + ((t0 + r) * p.H + h) * p.V + v0 + cc) =
-          __floats2bfloat162_rn(s.P[r][cc] * p.scale, s.P[r][cc + 1] * p.scale);
-  }
+}
+
+template <int NP, int STAGES>
+cudaError_t launch_state(const ChunkParams& p, cudaStream_t stream) {
+  static SmemOptIn opt;
+  constexpr int smem = StateLay<NP>::smem(STAGES);
+  const cudaError_t e = opt.ensure(gdn_chunk_state<NP, STAGES>, smem);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(gdn_chunk_state<NP, STAGES>, dim3(p.V / (16 * NP), p.H, p.N), dim3(kStateThreads), smem, stream, p);
+}
+template <int RB>
+cudaError_t launch_output(const ChunkParams& p, cudaStream_t stream) {
+  static SmemOptIn opt;
+  constexpr int smem = static_cast<int>(sizeof(OutSmem));
+  const cudaError_t e = opt.ensure(gdn_chunk_output<RB>, smem);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(gdn_chunk_output<RB>, dim3(p.NC, p.H), dim3(kThreads), smem, stream, p);
 }
 
 }  // namespace
 
 cudaError_t launch_gdn_chunk_fwd(const GdnChunkArgs& a, cudaStream_t stream) {
-  if (a.K != kK || a.V % 64 != 0 || a.V < 64 || a.V > 256 || a.num_seqs < 1 || a.num_chunks < 0) return cudaErrorInvalidValue;
-  if (a.num_chunks == 0) return cudaSuccess;
+  if (a.K != kK || a.V % 64 != 0 || a.V < 64 || a.V > 256 || a.num_seqs < 1 || a.num_chunks < 1) return cudaErrorInvalidValue;
   ChunkParams p;
   p.q = reinterpret_cast<const __nv_bfloat16*>(a.q);
   p.k = reinterpret_cast<const __nv_bfloat16*>(a.k);
   p.v = reinterpret_cast<const __nv_bfloat16*>(a.v);
   p.g = a.g;
   p.beta = reinterpret_cast<const __nv_bfloat16*>(a.beta);
-  p.cu_seqlens = a.cu_seqlens;
-  p.chunk_seq = a.chunk_seq;
-  p.chunk_t0 = a.chunk_t0;
-  p.seq_chunk0 = a.seq_chunk0;
+  p.cu = a.cu_seqlens;
+  p.chunk_seq = a.tables;
+  p.chunk_t0 = a.tables + a.num_chunks;
+  p.seq_chunk0 = a.tables + 2 * static_cast<int64_t>(a.num_chunks);
   p.gcum = a.g_cumsum;
   p.a_out = a.a_out;
-  p.w = reinterpret_cast<__nv_bfloat16*>(a.w);
-  p.u = reinterpret_cast<__nv_bfloat16*>(a.u);
-  p.vnew = reinterpret_cast<__nv_bfloat16*>(a.v_new);
-  p.hstate = reinterpret_cast<__nv_bfloat16*>(a.h_chunks);
+  p.decay = a.decay;
+  p.w = reinterpret_cast<uint4*>(a.w);
+  p.kd = reinterpret_cast<uint4*>(a.kd);
+  p.u = reinterpret_cast<uint4*>(a.u);
+  p.vnew = reinterpret_cast<uint4*>(a.v_new);
+  p.hstate = reinterpret_cast<uint4*>(a.h_chunks);
   p.h0 = a.initial_state;
   p.ht = a.final_state;
   p.o = reinterpret_cast<__nv_bfloat16*>(a.o);
-  p.H = a.H; p.V = a.V; p.NC = a.num_chunks;
+  p.H = a.H; p.V = a.V; p.N = a.num_seqs; p.NC = a.num_chunks;
   p.scale = a.scale;
-  static SmemOptIn opt1, opt2, opt3;
-  const int smem1 = static_cast<int>(sizeof(PrepSmem)) + kC * (a.V + 8) * 2;
-  const int smem2 = static_cast<int>(sizeof(StateSmem));
-  const int smem3 = static_cast<int>(sizeof(OutSmem));
-  cudaError_t e = opt1.ensure(gdn_chunk_prepare, 128 * 1024);
+  cudaError_t e = launch_pdl(gdn_chunk_tables, dim3(1), dim3(kThreads), 0, stream, p);
   if (e != cudaSuccess) return e;
-  e = opt2.ensure(gdn_chunk_state, smem2);
+  static SmemOptIn opt;
+  e = opt.ensure(gdn_chunk_prepare, 128 * 1024);
   if (e != cudaSuccess) return e;
-  e = opt3.ensure(gdn_chunk_output, smem3);
+  e = launch_pdl(gdn_chunk_prepare, dim3(a.num_chunks, a.H), dim3(kThreads), sizeof(PrepSmem) + kC * (a.V + 8) * 2, stream, p);
   if (e != cudaSuccess) return e;
-  if (smem1 > 128 * 1024) return cudaErrorInvalidValue;
-  gdn_chunk_prepare<<<dim3(a.num_chunks, a.H), kThreads, smem1, stream>>>(p);
-  e = cudaGetLastError();
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t ctas = static_cast<int64_t>(a.num_seqs) * a.H * (a.V / 16);
+  e = ctas <= sms ? launch_state<1, 5>(p, stream) : ctas <= 2 * sms ? launch_state<1, 3>(p, stream) : launch_state<2, 3>(p, stream);
   if (e != cudaSuccess) return e;
-  gdn_chunk_state<<<dim3(a.V / kVT, a.H, a.num_seqs), kThreads, smem2, stream>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  gdn_chunk_output<<<dim3(a.num_chunks, a.H, a.V / kVT), kThreads, smem3, stream>>>(p);
-  return cudaGetLastError();
+  return a.V == 64 ? launch_output<2>(p, stream) : launch_output<4>(p, stream);
 }
 
 }  // namespace tdb

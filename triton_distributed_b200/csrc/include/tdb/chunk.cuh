@@ -1,5 +1,5 @@
-// Pieces of the chunk-parallel recurrence kernels (gla_chunk.cu, delta_chunk.cu): fp32 operands as a high and a low bf16 part,
-// positions of the 64-token chunks, fragment loads.
+// Pieces of the chunk-parallel recurrence kernels (gla_chunk.cu, delta_chunk.cu, gdn_chunk.cu): fp32 operands as a high and a low bf16 part,
+// positions of the 64-token chunks, fragment loads, the triangular inverse.
 #pragma once
 #include "attn_device.cuh"
 #include "ptx.cuh"
@@ -8,6 +8,10 @@ namespace tdb {
 namespace chunk {
 
 constexpr int kC = 64;            // tokens per chunk
+constexpr int kFp = kC + 4;       // pitch of fp32 [64][64] matrices
+
+// Lower 16 x 16 block (bi, bj) of a 64 x 64 matrix.
+TDB_DEVICE constexpr int lower_block(int bi, int bj) { return bi * (bi + 1) / 2 + bj; }
 
 struct HiLo {
   uint32_t hi, lo;
@@ -48,6 +52,63 @@ TDB_DEVICE void load_tile(__nv_bfloat16* dst, int pitch, const __nv_bfloat16* sr
   for (int i = threadIdx.x; i < kC * vec; i += threads) {
     const int r = i / vec, c = i - r * vec;
     attn::cp_async16(dst + r * pitch + c * 8, src + (r < n ? r * ld : 0) + c * 8, r < n);
+  }
+}
+
+// A <- (I + A)^-1 for the strictly lower triangular A (blocks above the diagonal are scratch).
+template <int THREADS>
+TDB_DEVICE void invert_unit_lower(float* A) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp < 4) {                       // the 16 x 16 blocks on the diagonal by substitution, a column per lane
+    float* D = A + (warp * 16) * kFp + warp * 16;
+    float x[16];
+    const int j = lane & 15;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float a = (i == j) ? 1.f : 0.f, b = 0.f;
+#pragma unroll
+      for (int m = 0; m < i; ++m) {
+        if (m & 1) a = fmaf(-D[i * kFp + m], x[m], a);
+        else b = fmaf(-D[i * kFp + m], x[m], b);
+      }
+      x[i] = a + b;
+    }
+    __syncwarp();
+    if (lane < 16) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) D[i * kFp + j] = i >= j ? x[i] : 0.f;
+    }
+  }
+  __syncthreads();
+  // blocks below the diagonal, 16 then 32: A21 = -A22 (L21 A11); the product in brackets goes to the block above the diagonal.
+  // A thread owns four neighbouring columns of a row.
+#pragma unroll
+  for (int n = 16; n <= 32; n *= 2) {
+    const int per = n * n / 4, all = 32 / n * per;
+    for (int i = tid; i < all; i += THREADS) {
+      const int b = (i / per) * 2 * n, r = (i % per) / (n / 4), c = (i % (n / 4)) * 4;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int m = c & ~15; m < n; ++m) {
+        const float l = A[(b + n + r) * kFp + b + m];
+        const float4 v = *reinterpret_cast<const float4*>(A + (b + m) * kFp + b + c);
+        a.x = fmaf(l, v.x, a.x); a.y = fmaf(l, v.y, a.y); a.z = fmaf(l, v.z, a.z); a.w = fmaf(l, v.w, a.w);
+      }
+      *reinterpret_cast<float4*>(A + (b + r) * kFp + b + n + c) = a;
+    }
+    __syncthreads();
+    for (int i = tid; i < all; i += THREADS) {
+      const int b = (i / per) * 2 * n, r = (i % per) / (n / 4), c = (i % (n / 4)) * 4;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int m = 0; m < (r & ~15) + 16; ++m) {
+        const float l = -A[(b + n + r) * kFp + b + n + m];
+        const float4 v = *reinterpret_cast<const float4*>(A + (b + m) * kFp + b + n + c);
+        a.x = fmaf(l, v.x, a.x); a.y = fmaf(l, v.y, a.y); a.z = fmaf(l, v.z, a.z); a.w = fmaf(l, v.w, a.w);
+      }
+      *reinterpret_cast<float4*>(A + (b + n + r) * kFp + b + c) = a;
+    }
+    __syncthreads();
   }
 }
 

@@ -8,7 +8,7 @@ Per head the state ``S`` [K, V] follows ``S <- exp(g_t) S;  v' = beta_t (v_t - S
 o_t = scale S^T q_t``.  Three implementations of the same function live here:
 
 * ``csrc/gdn_chunk.cu``: the chunk-parallel WY form the reference uses (triangular solve per 64-token chunk,
-  sequential pass over chunk states, output pass) as three CUDA kernels with tensor-core products - the default for
+  sequential pass over chunk states, output pass) as CUDA kernels with tensor-core products - the default for
   bf16 CUDA tensors with K = 128 and V a multiple of 64, also the source of the per-chunk ``A`` matrices;
 * ``csrc/gdn.cu``: one CUDA kernel that walks the tokens with the state in registers (``impl="recurrent"``; other V);
 * ``gated_delta_rule_chunked``: the same chunked form with batched PyTorch ops - the CPU path;
@@ -129,11 +129,10 @@ def chunk_gated_delta_rule_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     if chunk_ok:
         lib = _native.load(True)
         cu = cu_seqlens.to(device=q.device, dtype=torch.int32).contiguous()
-        chunk_seq, chunk_t0, seq_chunk0 = _chunk_tables(cu_seqlens, q.device)
         o, gc, A, ht = lib.gdn_chunk_fwd(q[0].contiguous(), k[0].contiguous(), v[0].contiguous(), g[0].float().contiguous(),
                                          beta[0].to(torch.bfloat16).contiguous(), float(scale),
                                          initial_state.float().contiguous() if initial_state is not None else None,
-                                         bool(output_final_state), cu, chunk_seq, chunk_t0, seq_chunk0, bool(return_A))
+                                         bool(output_final_state), cu, bool(return_A))
         return gc.unsqueeze(0), o.unsqueeze(0), (A.unsqueeze(0) if return_A else None), (ht if output_final_state else None)
     if not recurrent_ok:
         gc, o, A, ht = gated_delta_rule_chunked(q, k, v, g, beta, scale, initial_state, cu_seqlens)
@@ -147,19 +146,6 @@ def chunk_gated_delta_rule_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     # chunk-local cumulative decay, cheap enough in torch: cumsum over T minus the value at each chunk start
     gc = _chunk_local_cumsum(g[0].float(), cu_seqlens)
     return gc.unsqueeze(0), o.unsqueeze(0), None, (ht if output_final_state else None)
-
-
-def _chunk_tables(cu_seqlens: torch.Tensor, device, chunk: int = CHUNK):
-    """Per chunk: its sequence and first token; per sequence: its first chunk (int32 device tensors)."""
-    cu = cu_seqlens.tolist()
-    seq_of, t0_of, first = [], [], [0]
-    for s in range(len(cu) - 1):
-        for t in range(cu[s], cu[s + 1], chunk):
-            seq_of.append(s)
-            t0_of.append(t)
-        first.append(len(seq_of))
-    mk = lambda x: torch.tensor(x, dtype=torch.int32, device=device)   # noqa: E731
-    return mk(seq_of), mk(t0_of), mk(first)
 
 
 def _chunk_local_cumsum(g: torch.Tensor, cu_seqlens: torch.Tensor, chunk: int = CHUNK) -> torch.Tensor:
