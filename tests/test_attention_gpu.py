@@ -36,6 +36,29 @@ def test_decode_split_kv(cfg):
         torch.testing.assert_close(lse, ref_lse.t().contiguous(), rtol=1e-2, atol=1e-2)
 
 
+@pytest.mark.parametrize("D,group,page", [(64, 1, 1), (64, 16, 0), (128, 17, 24), (128, 3, 64), (256, 5, 0), (256, 2, 16)])
+@pytest.mark.parametrize("splits", [-1, 1, 5, 32])
+def test_decode_token_edges(D, group, page, splits):
+    # a warp's 16 tokens, a block's 64, pages that end inside both, sequences without a token; one page per sequence (page 0) and many
+    from triton_distributed_b200.ops import attention_reference, dense_block_table, gqa_fwd_batch_decode
+
+    lens = [1, 15, 16, 17, 63, 64, 65, 0, 511]
+    B, Hkv = len(lens), 2
+    k, v, bt = _paged_cache(B, max(lens), Hkv, D, page or max(lens))
+    if page == 0:
+        bt = dense_block_table(B, "cuda")
+    q = torch.randn(B, group * Hkv, D, device="cuda", dtype=torch.bfloat16)
+    kv_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    cu = torch.arange(B + 1, dtype=torch.int32, device="cuda")
+    keep = [i for i, n in enumerate(lens) if n]
+    ref = attention_reference(q.float(), k.float(), v.float(), bt, cu, kv_lens, None, False)
+    out = gqa_fwd_batch_decode(q, k, v, None, None, kv_lens, bt, kv_split=splits)
+    torch.cuda.synchronize()
+    assert out[7].abs().max() == 0
+    # probabilities and output are rounded to bf16: 2^-9 each of sums of values of order one
+    torch.testing.assert_close(out[keep].float(), ref[keep].float(), rtol=2 ** -7, atol=2 ** -7)
+
+
 def test_decode_softcap():
     from triton_distributed_b200.ops import attention_reference, gqa_fwd_batch_decode
 

@@ -112,6 +112,34 @@ TDB_DEVICE void load_kv_block(const PagedKV& kv, int b, int h, int t0, int kv_en
   }
 }
 
+// One warp's part of a block: 16 tokens from t0 to the rows at sK / sV.  Lane l looks up the cache row of token l % 16, so a
+// page is found once per token and not once per 16 bytes.
+template <int D, bool TIED>
+TDB_DEVICE void load_kv_warp(const PagedKV& kv, int b, int h, int t0, int kv_end, uint8_t* sK, uint8_t* sV, float* sc, int64_t row0) {
+  constexpr int kChunksPerRow = D / 8;
+  constexpr int kPitch = Tiles<D>::kPitch;
+  const int lane = lane_id();
+  const int mine = t0 + (lane & 15);
+  int64_t row = 0;
+  if (mine < kv_end) {
+    if constexpr (TIED) row = row0 + mine;
+    else row = kv.max_pages == 1 ? row0 + mine : kv.token_row(b, mine);
+  }
+  const int64_t off = (row * kv.Hkv + h) * D;
+#pragma unroll
+  for (int i = 0; i < kChunksPerRow / 2; ++i) {
+    const int c = i * 32 + lane;
+    const int r = c / kChunksPerRow, ch = c - r * kChunksPerRow;
+    const int64_t src = __shfl_sync(0xffffffffu, off, r) + ch * 8;
+    const bool valid = t0 + r < kv_end;
+    cp_async16(sK + r * kPitch + ch * 16, kv.k + src, valid);
+    if constexpr (!TIED) cp_async16(sV + r * kPitch + ch * 16, kv.v + src, valid);
+  }
+  if constexpr (TIED) {
+    if (lane < 16) cp_async4(sc + lane, kv.k_scale + row, mine < kv_end);
+  }
+}
+
 // Soft cap: scores -> cap * tanh(to_cap * score), to fp32 accuracy of the cap.  While all arguments of the warp are small the power
 // series of tanh takes the place of an exponential and a division, which the softmax's own exponentials would have to share a unit
 // with.  Executed by whole warps.
@@ -319,32 +347,34 @@ TDB_DEVICE void decode_splitkv_body(const DecodeParams& p, int split, int yidx, 
   w.load_q(h_lo < p.group ? qb + static_cast<int64_t>(head0 + h_lo) * D : nullptr,
            h_hi < p.group ? qb + static_cast<int64_t>(head0 + h_hi) * D : nullptr);
   const int nblk = blk1 - blk0;
-  const int64_t row0 = TIED ? p.kv.token_row(b, 0) : 0;
+  const int64_t row0 = (TIED || p.kv.max_pages == 1) && kv_len > 0 ? p.kv.token_row(b, 0) : 0;
+  // A warp takes 16 of a block's 64 tokens, fetches them itself and waits for nobody else until the merge: the stream is
+  // bound by HBM, and with blocks fetched by the whole CTA every warp waited twice per block for the slowest.
+  auto fetch = [&](int i) {
+    uint8_t* nK = smem + (i % S) * stage_bytes<D, TIED>();
+    const int r = warp * 16;
+    load_kv_warp<D, TIED>(p.kv, b, hkv, (blk0 + i) * kBlockN + r, kv_len, nK + r * T::kPitch, nK + T::kTileBytes + r * T::kPitch,
+                          reinterpret_cast<float*>(nK + T::kTileBytes) + r, row0);
+  };
   // one commit group per block, empty when there is no block left, so that "all but the newest S - 1 groups are
   // complete" always means "block i has landed"
 #pragma unroll
   for (int j = 0; j < S - 1; ++j) {
-    if (j < nblk) {
-      uint8_t* nK = smem + j * stage_bytes<D, TIED>();
-      load_kv_block<D, TIED>(p.kv, b, hkv, (blk0 + j) * kBlockN, kv_len, nK, nK + T::kTileBytes, row0);
-    }
+    if (j < nblk) fetch(j);
     cp_async_commit();
   }
   for (int i = 0; i < nblk; ++i) {
     uint8_t* sK = smem + (i % S) * stage_bytes<D, TIED>();
     uint8_t* sV = TIED ? sK : sK + T::kTileBytes;
-    if (i + S - 1 < nblk) {
-      uint8_t* nK = smem + ((i + S - 1) % S) * stage_bytes<D, TIED>();
-      load_kv_block<D, TIED>(p.kv, b, hkv, (blk0 + i + S - 1) * kBlockN, kv_len, nK, nK + T::kTileBytes, row0);
-    }
+    if (i + S - 1 < nblk) fetch(i + S - 1);
     cp_async_commit();
     cp_async_wait<S - 1>();
-    sync();
-    // each warp takes 16 of the block's 64 tokens
+    __syncwarp();
     w.template step<2, TIED>(sK, sV, (blk0 + i) * kBlockN, warp * 16, kv_len, kv_len, p.scale, p.softcap,
                              reinterpret_cast<const float*>(sK + T::kTileBytes));
-    sync();
+    __syncwarp();
   }
+  sync();       // the merge reuses the stages
   // merge the 4 warps (different token subsets, same rows) through shared memory
   float inv[2], lse[2];
   w.finish(inv, lse);
@@ -355,6 +385,7 @@ TDB_DEVICE void decode_splitkv_body(const DecodeParams& p, int split, int yidx, 
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int row = g + 8 * r;
+    if (hc * 16 + row >= p.group) continue;
 #pragma unroll
     for (int jd = 0; jd < D / 8; ++jd) {
       red_o[(warp * 16 + row) * D + 8 * jd + c] = w.o[jd][2 * r];

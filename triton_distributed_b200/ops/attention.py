@@ -122,16 +122,18 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 
 
 def pick_kv_splits(batch: int, num_kv_heads: int, head_dim_chunks: int, max_kv_len: int, num_sms: int = 148) -> int:
-    """Number of KV splits.  A CTA walks its 64-token blocks one after the other (about a microsecond each) and the
-    merge of the partials grows with the number of splits (about a tenth of that per split), so a small problem takes
-    about sqrt(8 x blocks) splits; a large batch is limited to what still fits one wave of the grid (three CTAs of
-    the split-KV kernel are resident per SM; a second, partly filled wave costs more than the extra parallelism
-    brings).  At most 64."""
+    """Number of KV splits: the larger of two wants.  While one CTA per SM is not reached, as many splits as that takes, down to a
+    single 64-token block each (4 sequences x 4 heads x 512 tokens: 5.7 us with 8 splits, 7.2 with 2).  Beyond, splits of at least
+    four blocks up to three waves of the three CTAs an SM holds: the last wave and sequences of unequal length cost less when the
+    pieces are small, the merge more (64 x 8 heads x 4096 tokens: 148 us with 1 split, 132 with 3, 139 with 6; 8 x 4 x 2048: 20.0 us
+    with 3, 13.9 with 8, 17.5 with 16).  Above 32 the merge is a launch of its own (1 x 8 x 32768: 30.6 us with 32 splits, 38 with
+    55), worth it only where 32 splits leave SMs idle.  At most 64."""
     blocks = max(1, (max_kv_len + 63) // 64)
     ctas = max(1, batch * num_kv_heads * head_dim_chunks)
-    one_wave = max(1, (3 * num_sms) // ctas)
-    want = max(1, math.ceil(math.sqrt(8.0 * blocks)))
-    return int(max(1, min(want, one_wave, blocks, 64)))
+    one_each = min(blocks, num_sms // ctas)
+    waves = min(blocks // 4, (9 * num_sms + ctas // 2) // ctas)
+    cap = FUSED_COMBINE_MAX_SPLITS if ctas * FUSED_COMBINE_MAX_SPLITS >= num_sms else 64
+    return max(1, min(max(one_each, waves), cap))
 
 
 FUSED_COMBINE_MAX_SPLITS = 32   # up to here the last split CTA merges the partials itself; beyond, a combine launch
