@@ -179,3 +179,20 @@ def test_gemv_fused(M, mode):
             torch.cuda.synchronize()
             err = (buf.float() - ref).abs().max().item() / (ref.abs().max().item() + 1e-6)
             assert err < 2e-2, f"gemv in-place {mode} M={M} N={N} K={K}: rel err {err}"
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (2, 1, 40), (1, 149, 264), (3, 4096, 1000), (5, 1185, 2056), (1, 20011, 520), (8, 151, 8192),
+                                   (16, 4099, 6112), (1, 300, 98272)])
+def test_gemv_spans(M, N, K):
+    # warps' spans that begin and end inside a group, groups with fewer rows, idle warps, every depth of the weight ring
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(N)
+    assert ops.gemv_supported(M, K)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    out = ops.gemv_fused(x, w).double()
+    torch.cuda.synchronize()
+    # one rounding to bf16 (2^-9 of the value) and fp32 sums of K products of order one over sqrt(K)
+    assert ((out - ref).abs() <= ref.abs() * 2 ** -8 + 2 ** -20 * K ** 0.5 + 1e-5).all()

@@ -2,9 +2,8 @@
 //
 // With so few tokens a linear layer is a pure weight stream: the tensor cores have nothing to amortise and the cost
 // of a decode step is the HBM time of the weights plus whatever each launch adds around it.  This kernel therefore
-// keeps the stream as plain as possible (every warp owns whole output columns, reads their weight rows with 16-byte
-// loads that stay many deep in flight, and reduces inside the warp, so there is no split-K, no atomics and no
-// second pass) and folds the neighbouring small kernels of a transformer layer into its prologue and epilogue:
+// keeps the stream as plain as possible (every warp owns an equal span of the CTA's weight rows, fetched in 16-byte
+// copies that stay many deep in flight, and sums on the tensor cores, so there are no atomics and no second pass) and folds the neighbouring small kernels of a transformer layer into its prologue and epilogue:
 //   prologue   f = RMSNorm(x) * g      (the sum of squares is taken while the activations are staged)
 //              f = SiLU(gate) * up     (x is the fused gate | up projection)
 //   epilogue   all-reduce of the result over the tensor-parallel ranks: every CTA publishes its columns in the
@@ -20,6 +19,7 @@
 
 #include <cstdlib>
 
+#include "tdb/attn_device.cuh"
 #include "tdb/gemv.h"
 #include "tdb/launch.cuh"
 #include "tdb/symm_device.cuh"
@@ -31,8 +31,11 @@ namespace {
 
 constexpr int kGemvThreads = 512;
 constexpr int kGemvWarps = kGemvThreads / 32;
-constexpr int kRedBytes = 8 * 1024;   // shared memory kept for the K-slice partial sums (32 slots of 8 x 8 floats)
+constexpr int kRedBytes = 2 * kGemvWarps * 256;   // partial sums of eight tokens: two parts per warp, 8 x 8 floats each
 constexpr int kMaxSmem = 200 * 1024;
+constexpr int kMinRing = kGemvWarps * 2 * 512;
+constexpr int kLaunchSmem = 225 * 1024;        // dynamic, beside at most 1.1 KB of static shared memory
+static_assert(kMaxSmem + kRedBytes + kMinRing <= kLaunchSmem, "what fits without a ring must fit with the smallest");
 
 struct GemvParams {
   int M, N, K;
@@ -79,18 +82,33 @@ TDB_DEVICE void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Work layout.  A CTA owns `rows_per_cta` (a multiple of 8) output columns = weight rows, in groups of 8.  A warp
-// takes one group and one slice of K; lane (g = lane / 4, t = lane % 4) streams row g of the group with 16-byte
+// Work layout.  A CTA owns `rows_per_cta` output columns = weight rows, in groups of 8 (the last one may be partly
+// empty).  The steps of all its groups, laid end to end, are cut into sixteen equal spans, one per warp, so that every
+// warp streams the same number of bytes whatever the shape: a span begins and ends anywhere inside a group, and a group
+// that several warps share is summed through shared memory at the end (a warp has at most two such parts: one that begins
+// inside its group, slot 2 warp, and one that begins with it, slot 2 warp + 1).  The kernel is bound by the weights'
+// HBM time; with whole groups per warp, SMs waited for the warps that had one group more.
+// Lane (g = lane / 4, t = lane % 4) streams row g of the group with 16-byte
 // loads, 32 elements of K per step across the four t lanes.  The dot products run on the tensor cores: the eight
 // loaded values of a lane are fed as the A fragments of two m16n8k16 steps (rows 8..15 of A are zero), the eight
 // activations of the same K positions of token g as the B fragments.  A dot product does not care in which order K
 // is walked, so the K positions are simply assigned to fragment slots in the order the 16-byte loads deliver them;
 // the accumulator then holds [8 rows x 8 tokens] and no lane-wise reduction is needed.  What is left per lane and
-// load is one shared-memory read and two mma instructions, so the warps spend their issue slots on keeping loads
-// in flight (kJ per lane, double buffered).  Slices of K are summed through shared memory at the end.
-constexpr int kJ = 8;
+// load is two shared-memory reads and two mma instructions.
+// The weights land in shared memory (cp.async), in a ring of R batches of J steps per warp that only the lane that fetched
+// a vector reads: no barrier.  Loads to registers need room in L1 while they are in flight, and next to attention kernels
+// that have the SM configured for shared memory there is next to none: inside a decode step the register form ran at half
+// the rate it had alone (lm_head of 151936 x 4096: 188 us alone and 240 to 410 us in the step; now 207 us in both.  gate | up of
+// 24576 x 4096 with one token: 71 us in the step, now 33).
+constexpr int kSpanSteps = 8;
 
-template <int MP>   // tokens rounded up to 1, 2, 4, 8 or 16 (two 8-token MMA tiles)
+// Steps of a warp when a CTA has `total`: whole batches, so that only a group's last batch is ever a partial one.
+TDB_DEVICE int warp_span(int total) {
+  const int per = (total + kGemvWarps - 1) / kGemvWarps;
+  return (per + kSpanSteps - 1) / kSpanSteps * kSpanSteps;
+}
+
+template <int MP, int J, int R>   // tokens rounded up to 1, 2, 4, 8 or 16 (two 8-token MMA tiles); ring
 __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams p) {
   extern __shared__ uint4 smem4[];
   __shared__ float s_part[kGemvWarps][MP];
@@ -101,34 +119,53 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   const int kv = p.K >> 3;                       // 16-byte vectors per row
   const int xs_stride = kv + 4;                  // in vectors: rows 64 bytes apart modulo 128 (bank-conflict free)
   uint4* xs = smem4;                             // staged activations f(x): [MP][xs_stride]
-  float* red = reinterpret_cast<float*>(smem4 + MP * xs_stride);   // [slots][8 rows][8 NT tokens] partial accumulators
+  uint4* ring = smem4 + MP * xs_stride + warp * (R * J * 32) + lane;                           // [R][J][32 lanes] of this warp
+  float* red = reinterpret_cast<float*>(smem4 + MP * xs_stride + kGemvWarps * R * J * 32);    // [2 per warp][8 rows][8 NT tokens]
   const int r0 = blockIdx.x * p.rows_per_cta;
   const int r1 = min(p.N, r0 + p.rows_per_cta);
-  const int groups = (r1 - r0 + 7) >> 3;         // groups this CTA really has (the last CTA may have fewer)
-  const int groups_nom = p.rows_per_cta >> 3;    // the warp layout follows the nominal count, the same in every CTA
-  const int slices = groups_nom >= kGemvWarps ? 1 : kGemvWarps / groups_nom;
-  const int steps_total = (kv + 3) >> 2;         // steps of 4 vectors (32 elements of K)
-
-  // this warp's first unit: (group, K slice)
-  int grp = slices == 1 ? warp : warp % groups_nom;
-  const int slice = slices == 1 ? 0 : warp / groups_nom;
-  const bool active = grp < groups && slice < slices;
-  const int st0 = (steps_total * slice) / slices, st1 = (steps_total * (slice + 1)) / slices;
+  const int groups = (r1 - r0 + 7) >> 3;
+  const int steps = (kv + 3) >> 2;               // steps of 4 vectors (32 elements of K) of a group
+  const int span = warp_span(groups * steps);
+  struct Seg {                                   // what is left of this warp's part of a group, and of its span behind st
+    int grp, st, end, left;
+  };
+  Seg cur;
+  cur.left = min(span, groups * steps - warp * span);
+  cur.grp = warp * span / steps;
+  cur.st = warp * span - cur.grp * steps;
+  cur.end = min(steps, cur.st + cur.left);
 
   // The weights do not depend on the previous kernel: the first loads are issued before anything else, so that
   // their latency overlaps the predecessor's tail (programmatic dependent launch) and the staging of x.
-  uint4 wa[kJ], wb[kJ];
-  auto issue = [&](uint4 (&dst)[kJ], int group, int step) {
-    const int row = min(r0 + group * 8 + g, p.N - 1);
-    const bool row_ok = r0 + group * 8 + g < r1;
-    const __nv_bfloat16* wr = p.w + static_cast<int64_t>(row) * p.ldw;
+  const int part0 = cur.st;      // where this warp's first part begins
+  const int grp0 = cur.grp;
+  auto fetch = [&](int slot, const Seg& s) {
+    if (s.left > 0) {
+      const int row = r0 + s.grp * 8 + g;
+      const bool row_ok = row < r1;
+      const __nv_bfloat16* wr = p.w + static_cast<int64_t>(row_ok ? row : r0) * p.ldw;
 #pragma unroll
-    for (int j = 0; j < kJ; ++j) {
-      const int c = (step + j) * 4 + t;
-      dst[j] = (row_ok && step + j < st1 && c < kv) ? ld_nc_v4(wr + c * 8) : make_uint4(0u, 0u, 0u, 0u);
+      for (int j = 0; j < J; ++j) {
+        const int c = (s.st + j) * 4 + t;
+        const bool ok = row_ok && s.st + j < s.end && c < kv;
+        attn::cp_async16(ring + (slot * J + j) * 32, wr + (ok ? c * 8 : 0), ok);
+      }
     }
+    attn::cp_async_commit();
   };
-  if (active) issue(wa, grp, st0);
+  // The batch behind `s`: of the same segment, or the first of the next group.
+  auto next = [&](const Seg& s) {
+    const int done = min(J, s.end - s.st);
+    Seg n{s.grp, s.st + done, s.end, s.left - done};
+    if (n.st == steps) n = Seg{s.grp + 1, 0, min(steps, n.left), n.left};
+    return n;
+  };
+  Seg ahead = cur;
+#pragma unroll
+  for (int i = 0; i < R - 1; ++i) {
+    fetch(i, ahead);
+    if (ahead.left > 0) ahead = next(ahead);
+  }
   pdl_wait();
   pdl_launch_dependents();
   // the call epoch is advanced by the last CTA of the previous call: read it only after the dependency wait
@@ -197,62 +234,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   __syncthreads();
 
   // ---- main loop
-  auto consume = [&](const uint4 (&src)[kJ], int step, float (&c)[NT][4]) {
-#pragma unroll
-    for (int j = 0; j < kJ; ++j) {
-      const int cv = (step + j) * 4 + t;
-      const bool in_range = step + j < st1 && cv < kv;
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const int tok = nt * 8 + g;               // token whose activations this lane feeds as the B fragment
-        uint4 xv = make_uint4(0u, 0u, 0u, 0u);
-        if (tok < MP && in_range) xv = xs[tok * xs_stride + cv];
-        mma_bf16_16816(c[nt], src[j].x, 0u, src[j].y, 0u, xv.x, xv.y);
-        mma_bf16_16816(c[nt], src[j].z, 0u, src[j].w, 0u, xv.z, xv.w);
-      }
-    }
-  };
-  if (active) {
-    for (; grp < groups; grp += kGemvWarps) {
-      float c[NT][4];
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-      int st = st0;
-      while (st < st1) {
-        // wa holds steps [st, st + kJ); fetch the next batch into wb before consuming wa, and vice versa
-        if (st + kJ < st1) issue(wb, grp, st + kJ);
-        consume(wa, st, c);
-        st += kJ;
-        if (st >= st1) break;
-        if (st + kJ < st1) issue(wa, grp, st + kJ);
-        consume(wb, st, c);
-        st += kJ;
-      }
-      // accumulator: c[0], c[1] = (row g, tokens 2t, 2t + 1); rows 8..15 of the tile are the zero half
-      const int slot = grp * slices + slice;
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        red[(slot * 8 + g) * (8 * NT) + nt * 8 + 2 * t] = c[nt][0];
-        red[(slot * 8 + g) * (8 * NT) + nt * 8 + 2 * t + 1] = c[nt][1];
-      }
-      const int nxt = grp + kGemvWarps;
-      if (slices == 1 && nxt < groups) issue(wa, nxt, st0);
-      if (slices != 1) break;
-    }
-  }
-  __syncthreads();
-
-  // ---- sum the K slices, scale, store
   __nv_bfloat16* pdst = nullptr;   // all-reduce: where this rank's partial result goes
   if (p.all_reduce)
     pdst = p.partial + par * p.partial_half + (p.use_mc ? 0ull : static_cast<uint64_t>(p.symm.rank) * p.m_cap * p.N);
-  for (int i = tid; i < groups * 8 * p.M; i += kGemvWarps * 32) {
-    const int m = i / (groups * 8), rr = i - m * (groups * 8);     // consecutive threads -> consecutive columns
-    const int row = r0 + rr;
-    if (row >= r1) continue;
-    const int gi = rr >> 3, gr = rr & 7;
-    float v = 0.f;
-    for (int sl = 0; sl < slices; ++sl) v += red[((gi * slices + sl) * 8 + gr) * (8 * NT) + m];
+  auto store = [&](int m, int row, float v) {
     v *= s_rstd[m];
     if (p.all_reduce) {
       pdst[static_cast<int64_t>(m) * p.N + row] = __float2bfloat16(v);
@@ -260,6 +245,61 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
       if (p.residual != nullptr) v += __bfloat162float(p.residual[static_cast<int64_t>(m) * p.ld_res + row]);
       p.out[static_cast<int64_t>(m) * p.ld_out + row] = __float2bfloat16(v);
     }
+  };
+  float acc[NT][4];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+  for (int i = 0; cur.left > 0; ++i) {
+    fetch((i + R - 1) % R, ahead);
+    if (ahead.left > 0) ahead = next(ahead);
+    attn::cp_async_wait<R - 1>();
+    const uint4* src = ring + (i % R) * J * 32;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int cv = (cur.st + j) * 4 + t;
+      const bool in_range = cur.st + j < cur.end && cv < kv;
+      const uint4 wv = src[j * 32];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int tok = nt * 8 + g;               // token whose activations this lane feeds as the B fragment
+        uint4 xv = make_uint4(0u, 0u, 0u, 0u);
+        if (tok < MP && in_range) xv = xs[tok * xs_stride + cv];
+        mma_bf16_16816(acc[nt], wv.x, 0u, wv.y, 0u, xv.x, xv.y);
+        mma_bf16_16816(acc[nt], wv.z, 0u, wv.w, 0u, xv.z, xv.w);
+      }
+    }
+    if (cur.st + J >= cur.end) {   // the part is complete: acc[0], acc[1] = (row g, tokens 2t, 2t + 1), rows 8..15 of the tile are zero
+      const bool from_start = cur.grp != grp0 || part0 == 0;
+      float* slot = red + ((2 * warp + (from_start ? 1 : 0)) * 8 + g) * (8 * NT) + 2 * t;
+      const int row = r0 + cur.grp * 8 + g;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int m = nt * 8 + 2 * t + e;
+          if (from_start && cur.end == steps) {        // the whole group
+            if (m < p.M && row < r1) store(m, row, acc[nt][e]);
+          } else {
+            slot[nt * 8 + e] = acc[nt][e];
+          }
+        }
+        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+      }
+    }
+    cur = next(cur);
+  }
+  attn::cp_async_wait<0>();
+  __syncthreads();
+
+  // ---- groups that several warps share: sum their parts
+  for (int i = tid; i < groups * 8 * p.M; i += kGemvThreads) {
+    const int m = i / (groups * 8), rr = i - m * (groups * 8);     // consecutive threads -> consecutive columns
+    const int gi = rr >> 3, gr = rr & 7;
+    const int w0 = gi * steps / span, w1 = ((gi + 1) * steps - 1) / span;
+    if (r0 + rr >= r1 || w0 == w1) continue;
+    float v = 0.f;
+    for (int w = w0; w <= w1; ++w) v += red[((2 * w + (w * span <= gi * steps ? 1 : 0)) * 8 + gr) * (8 * NT) + m];
+    store(m, r0 + rr, v);
   }
 
   // ---- epilogue: all-reduce of this CTA's columns [r0, r1) (multiples of 8) with the same CTA of every rank
@@ -330,16 +370,25 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   }
 }
 
+template <int M, int J, int R>
+cudaError_t launch_ring(const GemvParams& p, int grid, size_t smem, cudaStream_t stream) {
+  static SmemOptIn opt;
+  cudaError_t e = opt.ensure(gemv_kernel<M, J, R>, kLaunchSmem);
+  if (e != cudaSuccess) return e;
+  // everything the kernel reads from its predecessor comes after pdl_wait()
+  return launch_pdl(gemv_kernel<M, J, R>, dim3(grid), dim3(kGemvThreads), smem + kGemvWarps * J * R * 512, stream, p);
+}
+
+// The deepest ring that fits beside the activations and the partial sums (`smem` bytes).  40 KB per SM must be in flight to
+// cover HBM's latency: the 128 KB ring has 96 KB, the 16 KB one is what the largest activations leave.  Four steps a batch ask for
+// 256 bytes of a row at once: 4096 x 12288 takes 19.9 us, with two steps and eight batches 22.5, with eight and two 20.6.
 template <int M>
 cudaError_t launch_t(const GemvParams& p, int grid, size_t smem, cudaStream_t stream) {
-  static bool set = false;
-  if (!set) {
-    cudaError_t e = cudaFuncSetAttribute(gemv_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    if (e != cudaSuccess) return e;
-    set = true;
-  }
-  // everything the kernel reads from its predecessor comes after pdl_wait()
-  return launch_pdl(gemv_kernel<M>, dim3(grid), dim3(kGemvThreads), smem, stream, p);
+  const int left = kLaunchSmem - static_cast<int>(smem);
+  if (left >= kGemvWarps * 16 * 512) return launch_ring<M, 4, 4>(p, grid, smem, stream);
+  if (left >= kGemvWarps * 8 * 512) return launch_ring<M, 2, 4>(p, grid, smem, stream);
+  if (left >= kGemvWarps * 4 * 512) return launch_ring<M, 2, 2>(p, grid, smem, stream);
+  return launch_ring<M, 1, 2>(p, grid, smem, stream);
 }
 
 }  // namespace
@@ -379,8 +428,10 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   static_assert(sizeof(SymmInfo) == sizeof(SymmInfoHost), "SymmInfo mirrors must match");
   memcpy(&p.symm, &a.symm, sizeof(SymmInfo));
   const int num_ctas = a.num_ctas < 1 ? 1 : a.num_ctas;
-  // groups of 8 columns per warp; in all-reduce mode this also gives every CTA whole 16-byte vectors
-  const int rows = (((a.N + num_ctas - 1) / num_ctas) + 7) & ~7;
+  // As even as it goes: 4096 columns are 28 for each of 147 CTAs, not 32 for 128.  In all-reduce mode every CTA gets
+  // whole 16-byte vectors.
+  const int even = (a.N + num_ctas - 1) / num_ctas;
+  const int rows = a.all_reduce ? (even + 7) & ~7 : even;
   if (a.all_reduce) {
     // the residual / output rows must allow vector access
     if (a.N % 8 != 0 || a.ld_out % 8 != 0 || (a.residual != nullptr && a.ld_res % 8 != 0)) return cudaErrorInvalidValue;
@@ -390,10 +441,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   const int grid = (a.N + rows - 1) / rows;
   if (a.all_reduce && grid > a.max_ctas) return cudaErrorInvalidValue;
   const int mp = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : a.M <= 8 ? 8 : 16;
-  const int groups = rows / 8;
-  const int slots = groups >= kGemvWarps ? groups : groups * (kGemvWarps / groups);
-  const size_t smem = static_cast<size_t>(mp) * (a.K * 2 + 64) + static_cast<size_t>(slots) * 256 * ((mp + 7) / 8);
-  if (smem > static_cast<size_t>(kMaxSmem)) return cudaErrorInvalidValue;
+  const size_t smem = static_cast<size_t>(mp) * (a.K * 2 + 64) + static_cast<size_t>(kRedBytes) * ((mp + 7) / 8);
   switch (mp) {
     case 1: return launch_t<1>(p, grid, smem, stream);
     case 2: return launch_t<2>(p, grid, smem, stream);
