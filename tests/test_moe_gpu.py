@@ -120,3 +120,66 @@ def test_group_gemm_with_in_kernel_gather(rt, cfg):
     ok = sid >= 0
     torch.testing.assert_close(ys[ok].float(), ref[sid[ok]] * tw.reshape(-1)[sid[ok]].unsqueeze(-1), rtol=3e-2, atol=3e-2)
     assert (ys[: int(srt.meta[0])][~ok[: int(srt.meta[0])]] == 0).all()     # padding rows of visited tiles are zeros
+
+
+@pytest.mark.parametrize("n,E", [(0, 8), (1, 1), (8191, 128), (8193, 2048), (65536, 7), (65537, 128), (100, 2049)])
+def test_sort_sizes(n, E):
+    # both sides of the one-launch sort's limits; ids outside [0, E) are dropped, most experts of a large E are empty
+    from triton_distributed_b200.ops import sort_topk_ids_align_block_size
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.randint(-1, E + 1, (n, 1), device="cuda", dtype=torch.int32, generator=g)
+    s = sort_topk_ids_align_block_size(ids, E)
+    flat = ids.reshape(-1).long()
+    ok = (flat >= 0) & (flat < E)
+    counts = torch.bincount(flat[ok], minlength=E)
+    ends = ((counts + 127) // 128 * 128).cumsum(0)
+    assert torch.equal(s.counts.long(), counts) and torch.equal(s.offsets[1:].long(), ends) and s.offsets[0] == 0
+    assert s.meta.tolist() == [int(ends[-1]), int(ends[-1]) // 128]
+    want = torch.repeat_interleave(torch.arange(E, device="cuda"), (counts + 127) // 128)
+    assert torch.equal(s.tile_expert[:want.numel()].long(), want) and (s.tile_expert[want.numel():] == -1).all()
+    pos = s.pos_of[:n].long()
+    assert (pos[~ok] == -1).all() and torch.equal(s.sorted_ids[pos[ok]].long(), ok.nonzero().squeeze(1))
+    assert ((pos[ok] >= s.offsets[flat[ok]]) & (pos[ok] < s.offsets[flat[ok]] + counts[flat[ok]])).all()
+    assert int((s.sorted_ids >= 0).sum()) == int(ok.sum())
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(1, 4, 2, 64, 16), (130, 5, 3, 200, 136), (700, 8, 4, 256, 248), (257, 3, 1, 72, 384)])
+def test_gated_group_gemm_and_sorted_rows(rt, T, E, k, H, I):
+    # SwiGLU in the epilogue, then rows that are in sorted order already; widths that end inside a tile's halves
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(T)
+    x = torch.randn(T, H, device="cuda", dtype=torch.bfloat16)
+    w13 = (torch.randn(E, 2 * I, H, device="cuda") * H ** -0.5).to(torch.bfloat16)
+    w2 = (torch.randn(E, H, I, device="cuda") * I ** -0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)]).to(torch.int32)
+    rw = torch.rand(T, k, device="cuda")
+    srt = ops.sort_topk_ids_align_block_size(ids, E)
+    act = ops.group_gemm_gather(x, w13, srt, a_row_div=k, gated=True)
+    flat = ops.group_gemm_gather(x, w13, srt, a_row_div=k, gated=True, scatter_out=True)
+    y = ops.group_gemm_gather(act, w2, srt, a_row_div=0, row_weight=rw)
+    torch.cuda.synchronize()
+    pairs = ids.reshape(-1).long()
+    g, u = torch.einsum("pk,pnk->pn", x.double().repeat_interleave(k, 0), w13.double()[pairs]).chunk(2, -1)
+    ref = torch.nn.functional.silu(g) * u
+    pos = srt.pos_of.long()
+    # one rounding to bf16 of values of order one, and fp32 sums
+    torch.testing.assert_close(act[pos].double(), ref, rtol=2 ** -8, atol=2 ** -10)
+    torch.testing.assert_close(flat.double(), ref, rtol=2 ** -8, atol=2 ** -10)
+    ref2 = torch.einsum("pk,pnk->pn", act[pos].double(), w2.double()[pairs]) * rw.reshape(-1, 1).double()
+    torch.testing.assert_close(y[pos].double(), ref2, rtol=2 ** -8, atol=2 ** -10)
+    pad = srt.sorted_ids[:int(srt.meta[0])] < 0
+    assert act[:pad.numel()][pad].abs().max() == 0 if pad.any() else True
+
+
+@pytest.mark.parametrize("E", [1, 31, 128, 129, 512])
+def test_router_bf16_logits(E):
+    from triton_distributed_b200.ops import topk_router
+
+    logits = torch.randn(77, E, device="cuda").to(torch.bfloat16)
+    k = min(E, 6)
+    a, b = topk_router(logits, k), topk_router(logits.float(), k)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    p = torch.softmax(logits.double(), -1).gather(1, a[0].long())
+    torch.testing.assert_close(a[1].double(), p / p.sum(-1, keepdim=True), rtol=1e-5, atol=1e-7)

@@ -18,13 +18,14 @@ void check_cuda(cudaError_t e, const char* what) { TORCH_CHECK(e == cudaSuccess,
 int32_t* i32(at::Tensor& t) { return t.data_ptr<int32_t>(); }
 
 std::vector<at::Tensor> topk_router(const at::Tensor& logits, int64_t k, bool normalize) {
-  TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == at::kFloat && logits.dim() == 2 && logits.is_contiguous(),
-              "topk_router: contiguous fp32 [T, E] expected");
+  const bool bf16 = logits.scalar_type() == at::kBFloat16;
+  TORCH_CHECK(logits.is_cuda() && (bf16 || logits.scalar_type() == at::kFloat) && logits.dim() == 2 && logits.is_contiguous(),
+              "topk_router: contiguous fp32 or bf16 [T, E] expected");
   c10::cuda::CUDAGuard guard(logits.device());
   const int64_t T = logits.size(0), E = logits.size(1);
   at::Tensor ids = at::empty({T, k}, logits.options().dtype(at::kInt));
-  at::Tensor w = at::empty({T, k}, logits.options());
-  check_cuda(tdb::launch_topk_router(logits.data_ptr<float>(), i32(ids), w.data_ptr<float>(), T, E, k, normalize ? 1 : 0,
+  at::Tensor w = at::empty({T, k}, logits.options().dtype(at::kFloat));
+  check_cuda(tdb::launch_topk_router(logits.data_ptr(), bf16, i32(ids), w.data_ptr<float>(), T, E, k, normalize ? 1 : 0,
                                      cur_stream()),
              "launch_topk_router");
   return {ids, w};
@@ -176,12 +177,13 @@ std::vector<at::Tensor> moe_tile_schedule(const at::Tensor& sorted_ids, int64_t 
 void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor& w, const at::Tensor& sorted_ids,
                      const at::Tensor& tile_expert, const c10::optional<at::Tensor>& order, const at::Tensor& meta,
                      at::Tensor& y, int64_t k_top, int64_t a_row_div, bool scatter_out,
-                     const c10::optional<at::Tensor>& row_weight, int num_ctas) {
+                     const c10::optional<at::Tensor>& row_weight, int num_ctas, bool gated = false) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "moe_fused: bf16 x [rows, K]");
   TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.dim() == 3 && w.is_contiguous(), "moe_fused: bf16 w [E, N, K]");
   TORCH_CHECK(y.is_cuda() && y.scalar_type() == at::kBFloat16 && y.dim() == 2 && y.stride(1) == 1, "moe_fused: bf16 y");
   const int64_t K = x.size(1), E = w.size(0), N = w.size(1);
-  TORCH_CHECK(w.size(2) == K && y.size(1) == N, "moe_fused: shape mismatch");
+  TORCH_CHECK(w.size(2) == K && y.size(1) == (gated ? N / 2 : N) && (!gated || N % 2 == 0), "moe_fused: shape mismatch");
+  TORCH_CHECK(a_row_div > 0 || x.size(0) >= sorted_ids.numel(), "moe_fused: x must hold every sorted row");
   TORCH_CHECK(sorted_ids.scalar_type() == at::kInt && tile_expert.scalar_type() == at::kInt && meta.scalar_type() == at::kInt,
               "moe_fused: int32 index tensors expected");
   TORCH_CHECK(sorted_ids.numel() == tile_expert.numel() * 128, "moe_fused: sorted_ids must hold 128 rows per tile");
@@ -190,6 +192,7 @@ void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor
   g.x = x.data_ptr();
   g.ldx = x.stride(0);
   g.a_row_div = a_row_div;
+  g.gated = gated ? 1 : 0;
   g.sorted_ids = sorted_ids.data_ptr<int32_t>();
   g.tile_expert = tile_expert.data_ptr<int32_t>();
   if (order.has_value()) {
@@ -198,7 +201,7 @@ void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor
   }
   g.meta = meta.data_ptr<int32_t>();
   g.max_tiles = tile_expert.numel();
-  int r = tdb::encode_tensor_map_3d(&g.tmap_b, w.data_ptr(), tdb::kBF16, E, N, K, K * 2, static_cast<uint64_t>(N) * K * 2, 256, 64, 128);
+  int r = tdb::encode_tensor_map_3d(&g.tmap_b, w.data_ptr(), tdb::kBF16, E, N, K, K * 2, static_cast<uint64_t>(N) * K * 2, gated ? 128 : 256, 64, 128);
   TORCH_CHECK(r == 0, "tensor map (w) failed: ", r);
   g.y = y.data_ptr();
   g.ldy = y.stride(0);
@@ -215,10 +218,10 @@ void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor
 // Grouped GEMM with the rows gathered inside the kernel (single GPU): y = x[sorted_ids / a_row_div] @ w[expert]^T.
 void moe_group_gemm_gather(const at::Tensor& x, const at::Tensor& w, const at::Tensor& sorted_ids, const at::Tensor& tile_expert,
                            const c10::optional<at::Tensor>& order, const at::Tensor& meta, at::Tensor& y, int64_t k_top,
-                           int64_t a_row_div, bool scatter_out, const c10::optional<at::Tensor>& row_weight, int num_ctas) {
+                           int64_t a_row_div, bool scatter_out, const c10::optional<at::Tensor>& row_weight, int num_ctas, bool gated) {
   c10::cuda::CUDAGuard guard(x.device());
   tdb::MoeFusedArgs g;
-  fill_moe_common(g, x, w, sorted_ids, tile_expert, order, meta, y, k_top, a_row_div, scatter_out, row_weight, num_ctas);
+  fill_moe_common(g, x, w, sorted_ids, tile_expert, order, meta, y, k_top, a_row_div, scatter_out, row_weight, num_ctas, gated);
   g.mode = tdb::kMoePlain;
   check_cuda(tdb::launch_moe_fused(g, cur_stream()), "launch_moe_fused(plain)");
 }

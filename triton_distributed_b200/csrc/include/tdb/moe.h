@@ -8,8 +8,8 @@
 
 namespace tdb {
 
-// softmax over E router logits (fp32 [T, E]) and top-k: ids int32 [T, k], weights fp32 [T, k] (optionally renormalised).
-cudaError_t launch_topk_router(const float* logits, int32_t* ids, float* weights, int T, int E, int k, int normalize,
+// softmax over E router logits (fp32 or bf16 [T, E]) and top-k: ids int32 [T, k], weights fp32 [T, k] (optionally renormalised).
+cudaError_t launch_topk_router(const void* logits, bool bf16, int32_t* ids, float* weights, int T, int E, int k, int normalize,
                                cudaStream_t s);
 
 // Sort the n = T*k (token, slot) pairs by expert with every expert's rows padded to a multiple of `align`.
@@ -54,13 +54,14 @@ struct MoeFusedArgs {
   int K, N, k_top;
   const void* x;               // bf16 source rows [rows, ldx]; all-gather mode: the local token shard [t_local, ldx = K]
   int64_t ldx;
-  int a_row_div;               // source row of sorted row r = sorted_ids[r] / a_row_div
+  int a_row_div;               // source row of sorted row r = sorted_ids[r] / a_row_div; 0: row r itself (not all-gather)
+  int gated;                   // plain mode: w = gate rows then up rows, y [*, N / 2] = silu(gate) * up
   const int32_t* sorted_ids;   // [max_tiles * 128]
   const int32_t* tile_expert;  // [max_tiles]
   const int32_t* order;        // optional tile visiting order [max_tiles]
   const int32_t* meta;         // {padded rows, tiles}
   int max_tiles;
-  TensorMap tmap_b;            // weights [E][N][K], box [256 x 64], 128-byte swizzle
+  TensorMap tmap_b;            // weights [E][N][K], box [256 x 64] (gated: [128 x 64]), 128-byte swizzle
   void* y;                     // bf16 output rows [*, ldy]
   int64_t ldy;
   int scatter_out;             // 1: (token, slot) order, 0: sorted layout

@@ -23,6 +23,7 @@ import torch
 from .. import _native
 from ..runtime import Runtime, get_runtime
 from .common import new_ctx_dev, ref_all_gather, ref_all_reduce, ref_reduce_scatter, sm_count
+from .elementwise import silu_mul_reference
 
 BLOCK_M = 128
 
@@ -66,7 +67,9 @@ def moe_reduce_reference(y: torch.Tensor, w2: torch.Tensor, topk_ids: torch.Tens
 def topk_router(logits: torch.Tensor, k: int, normalize: bool = True):
     """softmax + top-k: int32 ids [T, k], fp32 weights [T, k]."""
     if _native.use_native(logits) and logits.shape[-1] <= 512 and k <= 32:
-        ids, w = _native.load(True).topk_router(logits.float().contiguous(), int(k), bool(normalize))
+        if logits.dtype != torch.bfloat16:
+            logits = logits.float()
+        ids, w = _native.load(True).topk_router(logits.contiguous(), int(k), bool(normalize))
         return ids, w
     return topk_router_reference(logits, k, normalize)
 
@@ -319,30 +322,35 @@ def group_gemm_sorted(a_sorted: torch.Tensor, w: torch.Tensor, srt: MoESort) -> 
 
 def group_gemm_gather(x: torch.Tensor, w: torch.Tensor, srt: MoESort, a_row_div: int, scatter_out: bool = False,
                       row_weight: Optional[torch.Tensor] = None, order: Optional[torch.Tensor] = None,
-                      out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      out: Optional[torch.Tensor] = None, gated: bool = False) -> torch.Tensor:
     """Grouped GEMM whose A rows are gathered inside the kernel: sorted row r multiplies ``x[sorted_ids[r] // a_row_div]``
-    (``a_row_div = k`` when ``x`` holds tokens, 1 when it holds (token, slot) pairs) with its tile's expert weight.
+    (``a_row_div = k`` when ``x`` holds tokens, 1 when it holds (token, slot) pairs, 0 when its row r already is sorted
+    row r) with its tile's expert weight.  ``gated``: ``w`` holds gate rows, then up rows, and the result is
+    ``silu(gate) * up`` [*, N / 2].
     Output in the sorted layout [cap, N], or in (token, slot) order [pairs, N] when ``scatter_out``; ``row_weight``
     [pairs] scales every row in the epilogue."""
     n_pairs = srt.pos_of.numel()
     rows = n_pairs if scatter_out else srt.sorted_ids.numel()
     if _native.use_native(x, w) and x.dtype == torch.bfloat16:
         if out is None:
-            out = torch.empty((rows, w.shape[1]), dtype=x.dtype, device=x.device)
+            out = torch.empty((rows, w.shape[1] // 2 if gated else w.shape[1]), dtype=x.dtype, device=x.device)
         rw = row_weight.reshape(-1).float().contiguous() if row_weight is not None else None
         _native.load(True).moe_group_gemm_gather(x, w.contiguous(), srt.sorted_ids, srt.tile_expert, order, srt.meta, out,
-                                                 int(srt.k), int(a_row_div), bool(scatter_out), rw, 0)
+                                                 int(srt.k), int(a_row_div), bool(scatter_out), rw, 0, bool(gated))
         return out
     ids = srt.sorted_ids.long()
     ok = ids >= 0
     a = torch.zeros((ids.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
-    a[ok] = x[ids[ok] // a_row_div]
-    y = group_gemm_sorted(a, w, srt).float()
+    a[ok] = x[ids[ok] // a_row_div] if a_row_div > 0 else x[ok.nonzero().squeeze(1)]
+    y = group_gemm_sorted(a, w, srt)
+    if gated:
+        y = silu_mul_reference(y)
+    y = y.float()
     if row_weight is not None:
         y[ok] = y[ok] * row_weight.reshape(-1).float()[ids[ok]].unsqueeze(-1)
     y = y.to(x.dtype)
     if scatter_out:
-        res = torch.zeros((rows, w.shape[1]), dtype=x.dtype, device=x.device)
+        res = torch.zeros((rows, y.shape[1]), dtype=x.dtype, device=x.device)
         res[ids[ok]] = y[ok]
         y = res
     if out is not None:
@@ -554,23 +562,14 @@ def _moe_reduce_fused(x, weights, chosen_experts, expert_weight, ctx: MoEReduceR
     x_sorted_layout = srt is not None
     if srt is None:
         srt = sort_topk_ids_align_block_size(chosen_experts, ctx.num_experts)
-    # sorted-layout input: row r of x IS sorted row r (identity gather through an iota index); pair-order input: gather
-    if x_sorted_layout:
-        ids = srt.sorted_ids
-        iota = torch.arange(ids.numel(), dtype=torch.int32, device=ids.device)
-        gather_ids = torch.where(ids >= 0, iota, ids)
-        w_rows = expert_weight.reshape(-1).float()[ids.clamp_min(0).long()]
-        srt_g = MoESort(gather_ids, srt.pos_of, srt.tile_expert, srt.offsets, srt.meta, srt.counts, srt.k)
-        row_weight = w_rows          # indexed by the gather id = sorted row
-    else:
-        srt_g = srt
-        row_weight = expert_weight.reshape(-1).float().contiguous()
+    a_row_div = 0 if x_sorted_layout else 1       # sorted-layout input: row r of x is sorted row r
+    row_weight = expert_weight.reshape(-1).float().contiguous()
     cap = srt.sorted_ids.numel()
     if ctx.y_sorted is None or ctx.y_sorted.shape[0] < cap or ctx.y_sorted.shape[1] != H:
         ctx.y_sorted = torch.empty((cap, H), dtype=x.dtype, device=x.device)
     y_sorted = ctx.y_sorted[:cap]
     if W == 1:
-        group_gemm_gather(x, weights, srt_g, a_row_div=1, scatter_out=False, row_weight=row_weight, out=y_sorted)
+        group_gemm_gather(x, weights, srt, a_row_div=a_row_div, scatter_out=False, row_weight=row_weight, out=y_sorted)
         return reduce_topk(y_sorted, srt, None, T)
     lib = _native.load(True)
     tiles_n = (H + 255) // 256
@@ -579,7 +578,7 @@ def _moe_reduce_fused(x, weights, chosen_experts, expert_weight, ctx: MoEReduceR
         ctx.ar_slots = rt.symm_tensor((2, W, ctx.max_token_num, H), x.dtype, zero=False)
     slots = ctx.ar_slots if all_reduce else ctx.rs_slots
     out = torch.empty((T if all_reduce else T // W, H), dtype=x.dtype, device=x.device)
-    lib.moe_group_gemm_reduce(rt.heap, x, weights.contiguous(), srt_g.sorted_ids, srt.tile_expert, srt.meta, y_sorted, int(k), 1,
+    lib.moe_group_gemm_reduce(rt.heap, x, weights.contiguous(), srt.sorted_ids, srt.tile_expert, srt.meta, y_sorted, int(k), a_row_div,
                               row_weight, srt.pos_of, int(T), ctx.chunk_done, slots, ctx.flags, ctx.ctx_dev, out,
                               int(n_chunks), int(ctx.n_red_ctas), bool(all_reduce), sm_count(x.device),
                               rt.config.wait_timeout_s)

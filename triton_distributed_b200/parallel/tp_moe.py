@@ -65,8 +65,7 @@ class TP_MoE:
         self.ag_ctx = self.rs_ctx = self.ll_ctx = None
 
     def _route(self, x: torch.Tensor):
-        logits = ops.gemm(x, self.router_w).float()
-        return ops.topk_router(logits, self.topk, self.norm_topk)
+        return ops.topk_router(ops.gemm(x, self.router_w), self.topk, self.norm_topk)
 
     def torch_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """Golden path.  x [T, H] replicated -> [T, H] replicated (partial sums all-reduced with NCCL / gloo)."""
@@ -96,8 +95,7 @@ class TP_MoE:
         """x [T, H] replicated -> [T, H] replicated (grouped GEMMs + all-reduce)."""
         ids, w = self._route(x)
         srt = ops.sort_topk_ids_align_block_size(ids, self.num_experts)
-        hs = ops.group_gemm_gather(x, self.w13, srt, a_row_div=self.topk)   # token rows gathered inside the GEMM
-        act = ops.silu_mul(hs)
+        act = ops.group_gemm_gather(x, self.w13, srt, a_row_div=self.topk, gated=True)   # token rows gathered inside the GEMM
         return ops.run_moe_reduce_ar(act, self.w2, ids, w, self.rs_ctx, sort=srt)
 
     def set_fwd(self, mode: str = "torch"):
