@@ -119,3 +119,33 @@ def test_prefill_both_kernels(cfg, impl):
         check_attention_errors()
         torch.testing.assert_close(out.float(), ref.float(), rtol=2e-2, atol=2e-2)
         torch.testing.assert_close(lse, ref_lse, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("cap,sink,causal", [(0.0, False, True), (0.0, True, False), (15.0, False, True)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("qlens,kvlens,pos0", [([2048], [2048], None), ([127, 128, 129, 255, 256, 257, 1, 513], [127, 640, 129, 300, 256, 1025, 385, 513], None),
+                                               ([700, 130], [900, 64], [200, 0]), ([640], [500], [-200])])
+def test_prefill_two_tiles(D, qlens, kvlens, pos0, cap, sink, causal):
+    # 256-row tiles of the tcgen05 kernel: rows, keys and causal edges on both sides of a tile and a block, tiles without a row or a
+    # key, rows that see nothing, row maxima that outgrow their reference
+    from triton_distributed_b200.ops import attention_reference, flash_attn_varlen
+    from triton_distributed_b200.ops.attention import check_attention_errors
+
+    torch.manual_seed(D)
+    B, Hq, Hkv = len(qlens), 16, 2
+    k, v, bt = _paged_cache(B, max(kvlens), Hkv, D, 48, seed=5)
+    k *= torch.linspace(0.1, 3.0, 48, device="cuda").to(k.dtype)[None, :, None, None]
+    q = torch.randn(sum(qlens), Hq, D, device="cuda", dtype=torch.bfloat16) * 2
+    cu = torch.tensor([0] + list(torch.tensor(qlens).cumsum(0)), dtype=torch.int32, device="cuda")
+    kv_lens = torch.tensor(kvlens, dtype=torch.int32, device="cuda")
+    qp = None if pos0 is None else torch.tensor(pos0, dtype=torch.int32, device="cuda")
+    sk = torch.randn(Hq, device="cuda") if sink else None
+    ref, ref_lse = attention_reference(q.float(), k.float(), v.float(), bt, cu, kv_lens, qp, causal, None, cap, True, sk)
+    out, lse = flash_attn_varlen(q, k, v, bt, cu, kv_lens, max(qlens), q_pos0=qp, causal=causal, softcap=cap, return_lse=True, impl="sm100", sink=sk)
+    torch.cuda.synchronize()
+    check_attention_errors()
+    # probabilities and output are rounded to bf16, 2^-9 each, in sums of values of order one
+    torch.testing.assert_close(out.float(), ref, rtol=2 ** -7, atol=2 ** -6)
+    seen = ref_lse > float("-inf")
+    assert torch.equal(lse > float("-inf"), seen)
+    torch.testing.assert_close(lse[seen], ref_lse[seen], rtol=1e-4, atol=1e-4)

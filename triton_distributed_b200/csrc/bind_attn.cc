@@ -109,11 +109,11 @@ std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k
                                         c10::optional<at::Tensor> q_pos0, int64_t max_q_len, int64_t max_kv_len, bool causal,
                                         double scale, c10::optional<at::Tensor> lse, c10::optional<at::Tensor> k_scale,
                                         c10::optional<at::Tensor> sink, c10::optional<at::Tensor> gate, double softcap) {
-  TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.scalar_type() == at::kBFloat16 && q.size(2) == 128,
-              "flash_fwd_sm100: q must be contiguous bf16 [T, Hq, 128]");
+  TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.scalar_type() == at::kBFloat16 && (q.size(2) == 128 || q.size(2) == 64),
+              "flash_fwd_sm100: q must be contiguous bf16 [T, Hq, 64 or 128]");
   TORCH_CHECK(k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.is_contiguous() &&
-                  v_cache.is_contiguous() && k_cache.size(3) == 128,
-              "flash_fwd_sm100: contiguous bf16 caches [pages, page, Hkv, 128]");
+                  v_cache.is_contiguous() && k_cache.size(3) == q.size(2),
+              "flash_fwd_sm100: contiguous bf16 caches [pages, page, Hkv, head dim of q]");
   check_i32(cu_seqlens_q, "cu_seqlens_q");
   check_i32(kv_lens, "kv_lens");
   check_i32(block_table, "block_table");
@@ -141,15 +141,15 @@ std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k
   a.max_q_len = max_q_len;
   a.num_q_heads = q.size(1);
   a.num_kv_heads = k_cache.size(2);
-  a.head_dim = 128;
+  a.head_dim = q.size(2);
   a.total_q = q.size(0);
   a.causal = causal ? 1 : 0;
   a.scale = scale;
   a.softcap = softcap;
   TORCH_CHECK(max_kv_len >= 1, "flash_fwd_sm100: max_kv_len must be positive");
   a.Lp = static_cast<int>((max_kv_len + 63) / 64 * 64);
-  at::Tensor kd = at::empty({a.batch * a.num_kv_heads, a.Lp, 128}, q.options());
-  at::Tensor vt = at::empty({a.batch * a.num_kv_heads, 128, a.Lp}, q.options());
+  at::Tensor kd = at::empty({a.batch * a.num_kv_heads, a.Lp, a.head_dim}, q.options());
+  at::Tensor vt = at::empty({a.batch * a.num_kv_heads, a.head_dim, a.Lp}, q.options());
   a.k_dense = kd.data_ptr();
   a.vt_dense = vt.data_ptr();
   a.error_flag = err.data_ptr<int32_t>();

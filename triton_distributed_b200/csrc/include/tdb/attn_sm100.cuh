@@ -48,6 +48,52 @@ struct TileCtx {
   int row0, rows_here, nblk;
 };
 
+// The end of a query row: COLS of its accumulators at tmem_o (zeros without any block), normalised, through sink and gate, to the columns
+// from col0 of the output row.  Executed by whole warps; only rows with row_ok write.
+template <int COLS>
+__device__ __forceinline__ void write_row(const FwdParams& p, uint32_t tmem_o, int col0, bool ok, bool any, bool row_ok, float m, float l,
+                                          int64_t tok, int head) {
+  if (!ok) return;
+  const float lse = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+  float inv = l > 0.f ? 1.f / l : 0.f;
+  if (p.epi.sink != nullptr && l > 0.f) inv /= 1.f + __expf(p.epi.sink[head] - lse);
+  const __nv_bfloat16* grow = p.epi.gate == nullptr ? nullptr
+                                                    : reinterpret_cast<const __nv_bfloat16*>(p.epi.gate) + tok * p.epi.ld_gate +
+                                                          static_cast<int64_t>(head) * p.dv + col0;
+  __nv_bfloat16* orow = p.out + (tok * p.Hq + head) * p.dv + col0;
+  tc_fence_after_sync();
+#pragma unroll
+  for (int c = 0; c < COLS; c += 32) {
+    uint32_t r[32];
+    if (any) {
+      tmem_ld_32x32(tmem_o + c, r);
+      tmem_ld_wait();
+    }
+    if (!row_ok) continue;
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) {
+      if (col0 + c + k >= p.dv) break;
+      uint4 gate = make_uint4(0u, 0u, 0u, 0u);
+      if (grow != nullptr) gate = *reinterpret_cast<const uint4*>(grow + c + k);
+      const uint32_t gw[4] = {gate.x, gate.y, gate.z, gate.w};
+      uint32_t out[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float x0 = any ? __uint_as_float(r[k + 2 * e]) : 0.f, x1 = any ? __uint_as_float(r[k + 2 * e + 1]) : 0.f;
+        if (grow != nullptr) {
+          const float2 z = unpack_bf16x2(gw[e]);
+          x0 *= 1.f / (1.f + __expf(-z.x));
+          x1 *= 1.f / (1.f + __expf(-z.y));
+        }
+        out[e] = pack_bf16x2(x0 * inv, x1 * inv);
+      }
+      *reinterpret_cast<uint4*>(orow + c + k) = make_uint4(out[0], out[1], out[2], out[3]);
+    }
+  }
+  tc_fence_before_sync();
+  if (row_ok && col0 == 0 && p.lse != nullptr) p.lse[static_cast<int64_t>(head) * p.total_q + tok] = lse;
+}
+
 // DV: columns of the output accumulator (a multiple of 32); the rows written have p.dv <= DV columns, a multiple of 8.  CAP: with
 // soft cap.
 template <int DV, bool CAP = false>
@@ -149,64 +195,9 @@ __device__ __forceinline__ void softmax_tile(const FwdParams& p, const TileCtx& 
     fence_proxy_async_smem();                     // P was written through the generic proxy, the MMA reads it through the async proxy
     mbar_arrive(p_full);
   }
-  float o[DV];
-#pragma unroll
-  for (int i = 0; i < DV; ++i) o[i] = 0.f;
-  if (ok && nblk > 0) {
-    if (!mbar_wait(pv_full, (nblk - 1) & 1, abort_flag, kWaitNs)) {
-      ok = false;
-    } else {
-      tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < DV / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_pv + lane_off + c * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c * 32 + i] = __uint_as_float(r[i]);
-      }
-      tc_fence_before_sync();
-    }
-  }
+  if (ok && nblk > 0 && !mbar_wait(pv_full, (nblk - 1) & 1, abort_flag, kWaitNs)) ok = false;
   if (!ok) *abort_flag = 1;
-  if (ok && row_ok) {
-    float inv = l > 0.f ? 1.f / l : 0.f;
-    const int64_t tok = static_cast<int64_t>(q_begin) + row0 + row;
-    if (p.epi.sink != nullptr && l > 0.f) {
-      const float lse = (m + log2f(l)) * 0.6931471805599453f;
-      inv /= 1.f + __expf(p.epi.sink[head] - lse);
-    }
-    if (p.epi.gate != nullptr) {
-      const uint4* g4 = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.epi.gate) +
-                                                       tok * p.epi.ld_gate + static_cast<int64_t>(head) * p.dv);
-#pragma unroll
-      for (int c = 0; c < DV / 8; ++c) {
-        if (8 * c >= p.dv) break;
-        const uint4 u = g4[c];
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 z = unpack_bf16x2(w[e]);
-          o[8 * c + 2 * e] *= 1.f / (1.f + __expf(-z.x));
-          o[8 * c + 2 * e + 1] *= 1.f / (1.f + __expf(-z.y));
-        }
-      }
-    }
-    __nv_bfloat16* orow = p.out + (tok * p.Hq + head) * p.dv;
-#pragma unroll
-    for (int c = 0; c < DV / 8; ++c) {
-      if (8 * c >= p.dv) break;
-      uint4 v;
-      v.x = pack_bf16x2(o[8 * c + 0] * inv, o[8 * c + 1] * inv);
-      v.y = pack_bf16x2(o[8 * c + 2] * inv, o[8 * c + 3] * inv);
-      v.z = pack_bf16x2(o[8 * c + 4] * inv, o[8 * c + 5] * inv);
-      v.w = pack_bf16x2(o[8 * c + 6] * inv, o[8 * c + 7] * inv);
-      *reinterpret_cast<uint4*>(orow + 8 * c) = v;
-    }
-    if (p.lse != nullptr)
-      p.lse[static_cast<int64_t>(head) * p.total_q + q_begin + row0 + row] =
-          l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
-  }
+  write_row<DV>(p, tmem_pv + lane_off, 0, ok, nblk > 0, row_ok, m, l, static_cast<int64_t>(q_begin) + row0 + row, head);
 }
 
 }  // namespace

@@ -69,8 +69,9 @@ def attention_reference(q, k_cache, v_cache, block_table, cu_seqlens_q, kv_lens,
     return out.to(q.dtype)
 
 
-TENSOR_CORE_DIMS = (64, 128, 256)      # head dims of the mma.sync kernels (tcgen05: 128)
+TENSOR_CORE_DIMS = (64, 128, 256)      # head dims of the mma.sync kernels (tcgen05: 64 and 128)
 SM100_PREFILL_MIN_Q = 128      # below this the 64-row mma.sync kernel has less padding and no KV packing pass
+SM100_PREFILL_MIN_Q_64 = 512   # heads of 64: 24 x 256 tokens 16.5 us against 12.4 of mma.sync, 512: 18.6 / 20.7, 8192: 323 / 1223
 _PENDING_ERRORS = []            # error flags of tcgen05 prefill launches that have not been looked at yet
 
 
@@ -92,7 +93,7 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     """Prefill / context attention.  ``q`` [T, Hq, D] packed; query row i of sequence b has absolute position
     ``q_pos0[b] + i`` (default: the queries are the last ``q_len`` positions of the ``kv_lens[b]`` visible tokens).
 
-    ``impl``: "auto" picks the tcgen05 kernel (head dim 128, positive scale, at least ``SM100_PREFILL_MIN_Q`` query rows per
+    ``impl``: "auto" picks the tcgen05 kernel (head dim 64 or 128, positive scale, at least ``SM100_PREFILL_MIN_Q`` query rows per
     sequence) and otherwise the ``mma.sync`` kernel; "sm100" / "mma" force one.  ``max_kv_len`` (an upper bound of
     ``kv_lens``) saves the tcgen05 path a device-to-host read.  ``softcap``: scores become ``softcap * tanh(score / softcap)``.
     ``sink`` fp32 [Hq]: exp(sink) joins every denominator (the LSE that is returned is that of the keys alone)."""
@@ -101,10 +102,10 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     if _native.use_native(q, k_cache, v_cache) and q.dtype == torch.bfloat16 and D in TENSOR_CORE_DIMS:
         lib = _native.load(True)
         lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=q.device) if return_lse else None
-        sm100_ok = D == 128 and scale > 0 and k_cache.dtype == torch.bfloat16 and os.environ.get("TDB200_ATTN_SM100", "1") != "0"
+        sm100_ok = D in (64, 128) and scale > 0 and k_cache.dtype == torch.bfloat16 and os.environ.get("TDB200_ATTN_SM100", "1") != "0"
         if impl == "sm100" and not sm100_ok:
-            raise ValueError("flash_attn_varlen: the tcgen05 kernel needs head dim 128, bf16 caches and a positive scale")
-        if impl == "sm100" or (impl == "auto" and sm100_ok and max_q_len >= SM100_PREFILL_MIN_Q):
+            raise ValueError("flash_attn_varlen: the tcgen05 kernel needs head dim 64 or 128, bf16 caches and a positive scale")
+        if impl == "sm100" or (impl == "auto" and sm100_ok and max_q_len >= (SM100_PREFILL_MIN_Q if D == 128 else SM100_PREFILL_MIN_Q_64)):
             if max_kv_len is None:
                 max_kv_len = int(kv_lens.max().item())
             out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous(),
