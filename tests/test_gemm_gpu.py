@@ -196,3 +196,19 @@ def test_gemv_spans(M, N, K):
     torch.cuda.synchronize()
     # one rounding to bf16 (2^-9 of the value) and fp32 sums of K products of order one over sqrt(K)
     assert ((out - ref).abs() <= ref.abs() * 2 ** -8 + 2 ** -20 * K ** 0.5 + 1e-5).all()
+
+
+@pytest.mark.parametrize("M,F,K", [(256, 256, 64), (257, 264, 200), (777, 520, 1024), (1024, 19 * 128, 128), (300, 5000, 72), (8, 384, 512)])
+def test_gemm_swiglu(M, F, K):
+    # gate and up columns that end inside a tile's halves, half-width tail tiles, rows that end inside a CTA's 128; few rows: two launches
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    g, u = (x.double() @ w.double().t()).chunk(2, dim=-1)
+    ref = torch.nn.functional.silu(g) * u
+    out = ops.gemm_swiglu(x, w)
+    torch.cuda.synchronize()
+    # one rounding to bf16 of values of order one behind fp32 sums; three roundings where gate and up are stored
+    torch.testing.assert_close(out.double(), ref, rtol=2 ** -8 if M >= 256 else 2 ** -6, atol=2 ** -10 if M >= 256 else 2 ** -8)

@@ -136,16 +136,17 @@ void* stats_ptr(const c10::optional<at::Tensor>& stats, int num_ctas) {
   return stats->data_ptr();
 }
 
-// C[M,N] = A[M,K] @ B[N,K]^T   (bf16)
+// C[M,N] = A[M,K] @ B[N,K]^T   (bf16); gated: b = gate rows then up rows, C[M,N/2] = silu(A gate^T) * (A up^T)
 void gemm_bf16(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, int block_n, int num_ctas,
-               const c10::optional<at::Tensor>& stats) {
+               const c10::optional<at::Tensor>& stats, bool gated) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && c.is_cuda(), "gemm: CUDA tensors expected");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && c.scalar_type() == at::kBFloat16,
               "gemm: bf16 expected");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm: 2-D tensors expected");
   TORCH_CHECK(a.stride(1) == 1 && b.stride(1) == 1 && c.stride(1) == 1, "gemm: innermost dimension must be contiguous");
   const int64_t M = a.size(0), K = a.size(1), N = b.size(0);
-  TORCH_CHECK(b.size(1) == K && c.size(0) == M && c.size(1) == N, "gemm: shape mismatch");
+  const int64_t cols = gated ? N / 2 : N;
+  TORCH_CHECK(b.size(1) == K && c.size(0) == M && c.size(1) == cols && (!gated || N % 16 == 0), "gemm: shape mismatch");
   TORCH_CHECK(K % 8 == 0 && a.stride(0) % 8 == 0 && b.stride(0) % 8 == 0, "gemm: K and row strides must be multiples of 8");
   if (M == 0 || N == 0) return;
   c10::cuda::CUDAGuard guard(a.device());
@@ -157,12 +158,13 @@ void gemm_bf16(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, int bloc
   g.ldc = c.stride(0);
   const bool tma_store_ok = c.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) == 0;
   g.cta_pair = pick_cta_pair(M, N, block_n, tma_store_ok) ? 1 : 0;
+  g.gated = gated ? 1 : 0;
   g.block_n = g.cta_pair ? 256 : pick_block_n(N, block_n);
   g.tmap_a = make_tmap3(a.data_ptr(), tdb::kBF16, 1, M, K, a.stride(0) * 2, a.stride(0) * 2 * M, 128, 64);
   g.tmap_b = make_tmap3(b.data_ptr(), tdb::kBF16, 1, N, K, b.stride(0) * 2, b.stride(0) * 2 * N,
                         g.cta_pair ? 128 : g.block_n, 64);
   if (tma_store_ok) {
-    g.tmap_c = make_tmap3(c.data_ptr(), tdb::kBF16, 1, M, N, c.stride(0) * 2, c.stride(0) * 2 * M, 128, 64);
+    g.tmap_c = make_tmap3(c.data_ptr(), tdb::kBF16, 1, M, cols, c.stride(0) * 2, c.stride(0) * 2 * M, 128, 64);
     g.use_tma_store = 1;
   }
   const int tile_m = g.cta_pair ? 256 : 128;
@@ -624,7 +626,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
 
   m.def("gemm_bf16", &gemm_bf16, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("block_n") = 0,
-        py::arg("num_ctas") = 0, py::arg("stats") = py::none());
+        py::arg("num_ctas") = 0, py::arg("stats") = py::none(), py::arg("gated") = false);
   m.def("ag_gemm_bf16", &ag_gemm_bf16, py::arg("heap"), py::arg("a_local"), py::arg("b"), py::arg("c"), py::arg("ws"),
         py::arg("flags"), py::arg("ctx"), py::arg("max_seg_rows"), py::arg("max_chunks"), py::arg("n_comm"),
         py::arg("block_n"), py::arg("num_ctas"), py::arg("use_multimem"), py::arg("timeout_s"),

@@ -76,6 +76,7 @@ struct GemmArgs {
   int use_tma_store;
   int block_n;      // 128 or 256
   int cta_pair;     // 1: CTA-pair kernel (256 x 256 tiles over two SMs); tmap_b then has a 128-row box
+  int gated;        // pair kernel, plain mode: b = gate rows then up rows, c [M, N / 2] = silu(gate) * up; tmap_c covers N / 2 columns
   int num_ctas;     // grid size (<= SM count)
   // fused modes
   int seg_rows;     // rows per rank segment (M = world * seg_rows)

@@ -87,19 +87,21 @@ class TP_MLP:
 
     def dist_triton_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """AG-GEMM -> SiLU*up -> GEMM-RS.  x [M/W, H] (row shard) -> [M/W, H] (row shard)."""
-        h = ops.ag_gemm(x, self.gate_up_proj, self.ag_ctx)
-        h = ops.silu_mul(h)
+        if self.world_size == 1:
+            h = ops.gemm_swiglu(x, self.gate_up_proj)
+        else:
+            h = ops.silu_mul(ops.ag_gemm(x, self.gate_up_proj, self.ag_ctx))
         return ops.gemm_rs(h, self.down_proj, self.rs_ctx)
 
     def dist_triton_AR_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """Own GEMMs + the all-reduce library; x replicated."""
-        h = ops.silu_mul(ops.gemm(x, self.gate_up_proj))
+        h = ops.gemm_swiglu(x, self.gate_up_proj)
         o = ops.gemm(h, self.down_proj)
         return ops.all_reduce(o, ctx=self.ar_ctx) if self.world_size > 1 else o
 
     def dist_triton_gemm_ar_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """GEMM -> act -> fused GEMM+AllReduce (decode sizes); x replicated."""
-        h = ops.silu_mul(ops.gemm(x, self.gate_up_proj))
+        h = ops.gemm_swiglu(x, self.gate_up_proj)
         return ops.gemm_allreduce_op(self.gemm_ar_ctx, h, self.down_proj)
 
     # per-op entry points used by the layer benchmarks of the reference (tp_mlp.py:231-274)
