@@ -223,6 +223,13 @@ void moe_group_gemm_gather(const at::Tensor& x, const at::Tensor& w, const at::T
   tdb::MoeFusedArgs g;
   fill_moe_common(g, x, w, sorted_ids, tile_expert, order, meta, y, k_top, a_row_div, scatter_out, row_weight, num_ctas, gated);
   g.mode = tdb::kMoePlain;
+  auto rows128 = [&](tdb::TensorMap* m, const at::Tensor& t) {
+    const uint64_t rows = t.size(0), pitch = t.stride(0) * 2;
+    return t.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 && t.stride(0) >= t.size(1) &&
+           tdb::encode_tensor_map_2d(m, t.data_ptr(), tdb::kBF16, rows, t.size(1), pitch, 128, 64, 128) == 0;
+  };
+  g.tma_x = a_row_div == 0 && rows128(&g.tmap_x, x);
+  g.tma_y = !scatter_out && y.size(0) >= sorted_ids.numel() && rows128(&g.tmap_y, y);
   check_cuda(tdb::launch_moe_fused(g, cur_stream()), "launch_moe_fused(plain)");
 }
 

@@ -62,6 +62,10 @@ struct MoeFusedArgs {
   const int32_t* meta;         // {padded rows, tiles}
   int max_tiles;
   TensorMap tmap_b;            // weights [E][N][K], box [256 x 64] (gated: [128 x 64]), 128-byte swizzle
+  // plain mode: what goes by TMA instead of through the gather warps (a_row_div = 0) and the epilogue's own stores (sorted layout)
+  int tma_x, tma_y;
+  TensorMap tmap_x;            // x, box [128 x 64], 128-byte swizzle
+  TensorMap tmap_y;            // y in the sorted layout, the same box
   void* y;                     // bf16 output rows [*, ldy]
   int64_t ldy;
   int scatter_out;             // 1: (token, slot) order, 0: sorted layout
