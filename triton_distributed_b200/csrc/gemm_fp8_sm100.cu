@@ -483,12 +483,17 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           const float scale = kb == 0 ? (scaled ? as_row[0] * bs_row[0] : 0.f) : scale_next;
           if (scaled && kb + 1 < num_kb) scale_next = as_row[kb + 1] * bs_row[kb + 1];
           const uint32_t t_part = tmem_base + b * kBN + half * 128 + (static_cast<uint32_t>(q * 32) << 16);
+          // 32 columns are on their way while the 32 before them are scaled and added, two at a time (4096 x 12288 x 4096: 309 us one
+          // after the other and one by one, 282 now)
+          const float2 scale2 = make_float2(scale, scale);
+          uint32_t r[2][32];
+          tmem_ld_32x32(t_part, r[0]);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32(t_part + c * 32, r);
             tmem_ld_wait();
-            if (c == 3) {
+            if (c < 3) {
+              tmem_ld_32x32(t_part + (c + 1) * 32, r[(c + 1) & 1]);
+            } else {
               // This warp has read its share of the partial buffer: hand it back to the tensor core.  The ordering
               // that matters (TMEM reads before the next MMA overwrites them) is carried by the tcgen05 fence, so the
               // arrival is relaxed: a release at cluster scope would make the warp wait for all of its outstanding
@@ -498,7 +503,12 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
               if (lane == 0) mbar_arrive_cluster_relaxed(b ? part_empty1 : part_empty0);
             }
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(r[j]), scale, acc[c * 32 + j]);
+            for (int j = 0; j < 32; j += 2) {
+              float* a2 = &acc[c * 32 + j];
+              const float2 x = fma2(make_float2(__uint_as_float(r[c & 1][j]), __uint_as_float(r[c & 1][j + 1])), scale2, make_float2(a2[0], a2[1]));
+              a2[0] = x.x;
+              a2[1] = x.y;
+            }
           }
         }
         if (!ok) break;
