@@ -212,3 +212,24 @@ def test_gemm_swiglu(M, F, K):
     torch.cuda.synchronize()
     # one rounding to bf16 of values of order one behind fp32 sums; three roundings where gate and up are stored
     torch.testing.assert_close(out.double(), ref, rtol=2 ** -8 if M >= 256 else 2 ** -6, atol=2 ** -10 if M >= 256 else 2 ** -8)
+
+
+@pytest.mark.parametrize("M,F,K", [(1, 4, 8), (1, 3, 264), (2, 1001, 520), (4, 12288, 256), (7, 149, 2048), (16, 300, 4096), (1, 70, 40000)])
+def test_gemv_swiglu(M, F, K):
+    # groups of four gate and four up rows: whole, shared by warps, partly empty
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(F)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    nw = (1.0 + 0.1 * torch.randn(K, device="cuda")).to(torch.bfloat16)
+    for norm in (None, nw):
+        xn = x.double()
+        if norm is not None:
+            xn = xn * torch.rsqrt(xn.pow(2).mean(-1, keepdim=True) + 1e-6) * norm.double()
+        g, u = (xn @ w.double().t()).chunk(2, dim=-1)
+        ref = torch.nn.functional.silu(g) * u
+        out = ops.gemv_fused(x, w, norm_weight=norm, eps=1e-6, swiglu=True)
+        torch.cuda.synchronize()
+        # one rounding to bf16 of values of order one behind fp32 sums; the normed activations are rounded to bf16 before them
+        torch.testing.assert_close(out.double(), ref, rtol=2 ** -8 if norm is None else 2 ** -6, atol=2 ** -10 if norm is None else 2 ** -6)

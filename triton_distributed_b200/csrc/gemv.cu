@@ -3,14 +3,18 @@
 // With so few tokens a linear layer is a pure weight stream: the tensor cores have nothing to amortise and the cost
 // of a decode step is the HBM time of the weights plus whatever each launch adds around it.  This kernel therefore
 // keeps the stream as plain as possible (every warp owns an equal span of the CTA's weight rows, fetched in 16-byte
-// copies that stay many deep in flight, and sums on the tensor cores, so there are no atomics and no second pass) and folds the neighbouring small kernels of a transformer layer into its prologue and epilogue:
+// copies that stay many deep in flight, and sums on the tensor cores, so there are no atomics and no second pass) and
+// folds the neighbouring small kernels of a transformer layer into its prologue and epilogue:
 //   prologue   f = RMSNorm(x) * g      (the sum of squares is taken while the activations are staged)
 //              f = SiLU(gate) * up     (x is the fused gate | up projection)
-//   epilogue   all-reduce of the result over the tensor-parallel ranks: every CTA publishes its columns in the
+//   epilogue   SiLU(gate) * up on the fp32 sums, where the product is a gate | up projection
+//              all-reduce of the result over the tensor-parallel ranks: every CTA publishes its columns in the
 //              symmetric heap, exchanges one epoch flag per peer with the CTA of the same index there, and reads the
 //              sum back with multimem.ld_reduce (or sums the peers' slots after a push when there is no multicast)
 //              residual add, in place if wanted
-// so a decoder layer is four GEMV launches plus attention.
+// so a decoder layer is four GEMV launches plus attention.  SwiGLU belongs to the epilogue of the first product: as a prologue every
+// CTA of the second one computed it for all K columns and all tokens (4096 x 12288, one token: 22.0 us
+// with it, 20.0 without; a decode step of four layers of an 8B model with three tokens: 652 us, now 602).
 //
 // Reference behaviour being matched (not its code): the decode path of layers/nvidia/tp_attn.py:160-213 and
 // tp_mlp.py:196-229 (rmsnorm -> linear -> ... -> linear -> all-reduce -> add) and the fused GEMM+AllReduce of
@@ -48,6 +52,7 @@ struct GemvParams {
   const __nv_bfloat16* norm_w;
   float eps;
   int gated;
+  int swiglu;                  // a group is four gate rows and the four up rows of the same output columns
   const __nv_bfloat16* residual;
   int64_t ld_res;
   int rows_per_cta;
@@ -121,9 +126,13 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   uint4* xs = smem4;                             // staged activations f(x): [MP][xs_stride]
   uint4* ring = smem4 + MP * xs_stride + warp * (R * J * 32) + lane;                           // [R][J][32 lanes] of this warp
   float* red = reinterpret_cast<float*>(smem4 + MP * xs_stride + kGemvWarps * R * J * 32);    // [2 per warp][8 rows][8 NT tokens]
+  const int cols = p.swiglu ? p.N >> 1 : p.N;    // of the output
   const int r0 = blockIdx.x * p.rows_per_cta;
-  const int r1 = min(p.N, r0 + p.rows_per_cta);
-  const int groups = (r1 - r0 + 7) >> 3;
+  const int r1 = min(cols, r0 + p.rows_per_cta);
+  const int gshift = p.swiglu ? 2 : 3;           // log2 of the output columns of a group
+  const int groups = (r1 - r0 + (1 << gshift) - 1) >> gshift;
+  const int gcol = g & ((1 << gshift) - 1);      // this lane's column of a group, its weight row lies up_off further
+  const int up_off = g >> gshift ? cols : 0;
   const int steps = (kv + 3) >> 2;               // steps of 4 vectors (32 elements of K) of a group
   const int span = warp_span(groups * steps);
   struct Seg {                                   // what is left of this warp's part of a group, and of its span behind st
@@ -141,9 +150,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   const int grp0 = cur.grp;
   auto fetch = [&](int slot, const Seg& s) {
     if (s.left > 0) {
-      const int row = r0 + s.grp * 8 + g;
+      const int row = r0 + (s.grp << gshift) + gcol;
       const bool row_ok = row < r1;
-      const __nv_bfloat16* wr = p.w + static_cast<int64_t>(row_ok ? row : r0) * p.ldw;
+      const __nv_bfloat16* wr = p.w + static_cast<int64_t>(row_ok ? row + up_off : r0) * p.ldw;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int c = (s.st + j) * 4 + t;
@@ -237,8 +246,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   __nv_bfloat16* pdst = nullptr;   // all-reduce: where this rank's partial result goes
   if (p.all_reduce)
     pdst = p.partial + par * p.partial_half + (p.use_mc ? 0ull : static_cast<uint64_t>(p.symm.rank) * p.m_cap * p.N);
-  auto store = [&](int m, int row, float v) {
+  auto store = [&](int m, int row, float v, float up) {
     v *= s_rstd[m];
+    if (p.swiglu) v = silu_f32(v) * (up * s_rstd[m]);
     if (p.all_reduce) {
       pdst[static_cast<int64_t>(m) * p.N + row] = __float2bfloat16(v);
     } else {
@@ -271,14 +281,15 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     if (cur.st + J >= cur.end) {   // the part is complete: acc[0], acc[1] = (row g, tokens 2t, 2t + 1), rows 8..15 of the tile are zero
       const bool from_start = cur.grp != grp0 || part0 == 0;
       float* slot = red + ((2 * warp + (from_start ? 1 : 0)) * 8 + g) * (8 * NT) + 2 * t;
-      const int row = r0 + cur.grp * 8 + g;
+      const int row = r0 + (cur.grp << gshift) + gcol;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int m = nt * 8 + 2 * t + e;
-          if (from_start && cur.end == steps) {        // the whole group
-            if (m < p.M && row < r1) store(m, row, acc[nt][e]);
+          if (from_start && cur.end == steps) {        // the whole group; an up row is 16 lanes from its gate row
+            const float up = p.swiglu ? __shfl_down_sync(0xffffffffu, acc[nt][e], 16) : 0.f;
+            if (m < p.M && row < r1 && up_off == 0) store(m, row, acc[nt][e], up);
           } else {
             slot[nt * 8 + e] = acc[nt][e];
           }
@@ -292,14 +303,19 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   __syncthreads();
 
   // ---- groups that several warps share: sum their parts
-  for (int i = tid; i < groups * 8 * p.M; i += kGemvThreads) {
-    const int m = i / (groups * 8), rr = i - m * (groups * 8);     // consecutive threads -> consecutive columns
-    const int gi = rr >> 3, gr = rr & 7;
+  const int shown = groups << gshift;
+  for (int i = tid; i < shown * p.M; i += kGemvThreads) {
+    const int m = i / shown, rr = i - m * shown;                   // consecutive threads -> consecutive columns
+    const int gi = rr >> gshift, gr = rr & ((1 << gshift) - 1);
     const int w0 = gi * steps / span, w1 = ((gi + 1) * steps - 1) / span;
     if (r0 + rr >= r1 || w0 == w1) continue;
-    float v = 0.f;
-    for (int w = w0; w <= w1; ++w) v += red[((2 * w + (w * span <= gi * steps ? 1 : 0)) * 8 + gr) * (8 * NT) + m];
-    store(m, r0 + rr, v);
+    float v = 0.f, up = 0.f;
+    for (int w = w0; w <= w1; ++w) {
+      const float* part = red + ((2 * w + (w * span <= gi * steps ? 1 : 0)) * 8 + gr) * (8 * NT) + m;
+      v += part[0];
+      if (p.swiglu) up += part[4 * 8 * NT];
+    }
+    store(m, r0 + rr, v, up);
   }
 
   // ---- epilogue: all-reduce of this CTA's columns [r0, r1) (multiples of 8) with the same CTA of every rank
@@ -415,6 +431,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   p.norm_w = reinterpret_cast<const __nv_bfloat16*>(a.norm_w);
   p.eps = a.eps;
   p.gated = a.gated;
+  p.swiglu = a.swiglu;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.ld_res = a.ld_res;
   p.all_reduce = a.all_reduce;
@@ -430,7 +447,9 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   const int num_ctas = a.num_ctas < 1 ? 1 : a.num_ctas;
   // As even as it goes: 4096 columns are 28 for each of 147 CTAs, not 32 for 128.  In all-reduce mode every CTA gets
   // whole 16-byte vectors.
-  const int even = (a.N + num_ctas - 1) / num_ctas;
+  if (a.swiglu && (a.N % 2 != 0 || a.all_reduce || a.residual != nullptr)) return cudaErrorInvalidValue;
+  const int cols = a.swiglu ? a.N / 2 : a.N;
+  const int even = (cols + num_ctas - 1) / num_ctas;
   const int rows = a.all_reduce ? (even + 7) & ~7 : even;
   if (a.all_reduce) {
     // the residual / output rows must allow vector access
@@ -438,7 +457,7 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
     if (a.ctx == nullptr || a.partial == nullptr || a.flags == nullptr || a.M > a.m_cap) return cudaErrorInvalidValue;
   }
   p.rows_per_cta = rows;
-  const int grid = (a.N + rows - 1) / rows;
+  const int grid = (cols + rows - 1) / rows;
   if (a.all_reduce && grid > a.max_ctas) return cudaErrorInvalidValue;
   const int mp = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : a.M <= 8 ? 8 : 16;
   const size_t smem = static_cast<size_t>(mp) * (a.K * 2 + 64) + static_cast<size_t>(kRedBytes) * ((mp + 7) / 8);

@@ -16,6 +16,7 @@ struct GemvArgs {
   const void* norm_w;   // bf16 [K] or null: f(x) = rmsnorm(x) * norm_w
   float eps;
   int gated;            // f(x) = act(x[:, :K]) * x[:, K:], 1: silu, 2: gelu (tanh form); 0: not gated
+  int swiglu;           // w = gate rows then up rows: out [M, N / 2] = silu(gate) * up (no residual, no all-reduce)
   const void* residual; // bf16 [M, ld_res] or null, added to the result; may be `out` itself
   int64_t ld_res;
   int num_ctas;

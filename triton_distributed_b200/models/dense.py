@@ -50,14 +50,14 @@ class DenseLLMLayer:
     def fwd_fused_decode(self, stream: torch.Tensor, position_ids, kv_cache, gemv_ctx):
         """Decode step for up to eight tokens with four fused GEMV launches plus attention: ``stream`` [M, H] holds
         the residual stream and is updated in place (norms in the GEMV prologues, all-reduce and residual add in
-        their epilogues, SiLU*up in the down projection's prologue)."""
+        their epilogues, SiLU*up in the epilogue of gate | up)."""
         a, m = self.attn, self.mlp
         bsz = stream.shape[0]
         qkv = ops.gemv_fused(stream, a.wqkv, norm_weight=self.input_norm_w, eps=self.eps)
         o = a._attend(qkv, position_ids, kv_cache, self.layer_idx, bsz, 1)
         ops.gemv_fused(o, a.wo, out=stream, residual=stream, ar_ctx=gemv_ctx)
-        gu = ops.gemv_fused(stream, m.gate_up_proj, norm_weight=self.post_norm_w, eps=self.eps)
-        ops.gemv_fused(gu, m.down_proj, out=stream, silu_mul=True, residual=stream, ar_ctx=gemv_ctx)
+        h = ops.gemv_fused(stream, m.gate_up_proj, norm_weight=self.post_norm_w, eps=self.eps, swiglu=True)
+        ops.gemv_fused(h, m.down_proj, out=stream, residual=stream, ar_ctx=gemv_ctx)
         return stream
 
 

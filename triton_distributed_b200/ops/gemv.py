@@ -18,7 +18,7 @@ import torch
 from .. import _native
 from ..runtime import Runtime, get_runtime
 from .common import new_ctx_dev, sm_count
-from .elementwise import GATED_ACTS, gated_act_reference
+from .elementwise import GATED_ACTS, gated_act_reference, silu_mul_reference
 
 GEMV_MAX_M = 16    # what the kernel accepts
 GEMV_FAST_M = 8    # up to here it beats the tcgen05 weight-streaming kernel (two MMA tiles of tokens are mma.sync-bound)
@@ -93,16 +93,22 @@ def gemv_supported(M: int, K: int) -> bool:
 
 def gemv_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                norm_weight: Optional[torch.Tensor] = None, eps: float = 1e-6, silu_mul: bool = False,
-               residual: Optional[torch.Tensor] = None, ar_ctx: Optional[GemvARContext] = None, act: str = "silu") -> torch.Tensor:
+               residual: Optional[torch.Tensor] = None, ar_ctx: Optional[GemvARContext] = None, act: str = "silu",
+               swiglu: bool = False) -> torch.Tensor:
     """``x`` [M<=16, K] (or [M, 2K] with ``silu_mul``), ``w`` [N, K] -> [M, N].  ``residual`` may be ``out`` itself.
     ``act``: what ``silu_mul`` applies to the gate columns ("silu", "gelu").
+    ``swiglu``: ``w`` [2 F, K] holds gate rows, then up rows, and the result is ``silu(gate) * up`` [M, F] (no residual, no ``ar_ctx``).
     With ``ar_ctx`` of a multi-rank runtime the per-rank results are summed over the ranks before the residual."""
     M = x.shape[0]
     N, K = w.shape
     do_ar = ar_ctx is not None and ar_ctx.world_size > 1
+    if swiglu and (residual is not None or do_ar):
+        raise ValueError("gemv_fused: swiglu has no residual and no all-reduce")
     if not (_native.use_native(x, w) and x.dtype == torch.bfloat16 and gemv_supported(M, K)):
         res = gemv_reference(x, w, norm_weight, eps, silu_mul, residual,
                              group=ar_ctx.rt.group if do_ar else None, all_reduce=do_ar, act=act)
+        if swiglu:
+            res = silu_mul_reference(res)
         if out is not None:
             out.copy_(res)
             return out
@@ -110,7 +116,7 @@ def gemv_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
     lib = _native.load(True)
     gated = 1 + GATED_ACTS[act] if silu_mul else 0
     if out is None:
-        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+        out = torch.empty((M, N // 2 if swiglu else N), dtype=x.dtype, device=x.device)
     if do_ar:
         if N != ar_ctx.N:
             raise ValueError(f"gemv_fused: N={N} differs from the context's N={ar_ctx.N}")
@@ -120,5 +126,5 @@ def gemv_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
                          bool(ar_ctx.use_multimem and rt.has_multicast), rt.config.wait_timeout_s)
         ar_ctx.calls += 1
     else:
-        lib.gemv_bf16(x, w, out, norm_weight, float(eps), gated, residual, 0)
+        lib.gemv_bf16(x, w, out, norm_weight, float(eps), gated, residual, 0, bool(swiglu))
     return out
