@@ -327,6 +327,14 @@ def test_delta_rule_prompts(rt, shape, impl, dtype):
     r.check()
 
 
+@pytest.mark.parametrize("shape", [(10, 5, 128, 128, 4), (13, 13, 64, 80, 3), (13, 1, 48, 176, 4), (20, 4, 16, 72, 2)])
+def test_delta_rule_many_heads(rt, shape):
+    # enough heads and columns for the wide tiles of the state pass, the last of them partly empty; sequences of one to three chunks
+    r = Rule(*shape, lens=[70, 1, 129, 64])
+    r.run([(s, 0, n) for s, n in enumerate(r.lens)], "chunk")
+    r.check()
+
+
 @pytest.mark.parametrize("shape", RULES)
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_delta_rule_portions_and_decoding(rt, shape, dtype):

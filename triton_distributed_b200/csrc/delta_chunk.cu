@@ -380,13 +380,23 @@ __global__ void __launch_bounds__(kThreads, 2) delta_local_kernel(const DeltaArg
 }
 
 // ---------------------------------------------------------------------------------------------------- sequential part
-// KS: 16-row blocks of dk, a warp each; NT: tiles of eight columns per CTA.
+// KS: 16-row blocks of dk, a warp each; NT: tiles of eight columns per CTA.  Every CTA of a head reads the whole of trans, which is
+// most of the traffic and what the pass is bound by: with 32 columns a CTA 96 heads of 128 x 128 over 6001 tokens moved 983 MB
+// from L2 in 259 us, with 64 columns 590 MB in 187.  A lane reads exactly the fragments it has copied, so trans waits in a ring of
+// two chunks of shared memory without a barrier (as registers it left no room for 64 columns).
+constexpr int kTransRing = 2;
+template <int KS, int NT>
+constexpr size_t state_smem() {
+  return static_cast<size_t>(2 * 2 * KS * 16 * (NT * 8 + 8) * 2) + (KS <= 8 ? static_cast<size_t>(kTransRing) * KS * KS * 64 * 16 : 0);
+}
+
 template <int KS, int NT>
 __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs p) {
   extern __shared__ __align__(16) uint8_t smem[];
   constexpr int kPitch = NT * 8 + 8;
-  constexpr bool kAhead = KS <= 8;          // the next chunk's operands wait in registers
+  constexpr bool kRing = KS <= 8;           // larger heads read trans where it lies
   constexpr int ksteps = KS;
+  constexpr int part = KS * 16 * kPitch;
   const int vtiles = p.dv >> 3;
   const int tile0 = blockIdx.x * NT, h = blockIdx.y, n = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3, mat = lane >> 3, mr = lane & 7;
@@ -394,7 +404,7 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
   pdl_wait();
   pdl_launch_dependents();
   __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(smem);       // [2][hi, lo][dk][pitch]
-  const int part = p.dk * kPitch;
+  uint4* ring = reinterpret_cast<uint4*>(smem + 2 * 2 * part * 2) + warp * ksteps * 64 + lane;       // [kTransRing][warp][ks][hi, lo][lane]
   float* st = p.state + ((static_cast<int64_t>(p.slots[n]) * p.H + h) * p.dk + warp * 16 + g) * p.dv + tile0 * 8 + 2 * t4;
   float S[NT][4];
 #pragma unroll
@@ -411,24 +421,28 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
   const float4* inject = reinterpret_cast<const float4*>(p.inject) + (static_cast<int64_t>(warp) * vtiles + tile0) * 32 + lane;
   uint4* states = reinterpret_cast<uint4*>(p.states) + (static_cast<int64_t>(warp) * vtiles + tile0) * 32 + lane;
   const int64_t tr_step = static_cast<int64_t>(ksteps) * ksteps * 64, in_step = static_cast<int64_t>(ksteps) * vtiles * 32;
-  uint4 nh[kAhead ? KS : 1], nl[kAhead ? KS : 1];
   float4 ni[NT] = {};
   float nd = 0.f;
-  auto fetch = [&](int c) {
+  auto fetch = [&](int c) {                 // inject to registers, a chunk ahead
+    if (c >= c1) return;
     const int64_t ch = static_cast<int64_t>(c) * p.H + h;
     nd = p.decay[ch];
-    if constexpr (kAhead) {
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        nh[ks] = trans[ch * tr_step + ks * 64];
-        nl[ks] = trans[ch * tr_step + ks * 64 + 32];
-      }
-    }
 #pragma unroll
     for (int j = 0; j < NT; ++j)
       if (j < tiles) ni[j] = inject[ch * in_step + j * 32];
   };
-  if (c0 < c1) fetch(c0);
+  auto copy = [&](int c) {                  // trans to the ring, one group per chunk
+    if (kRing && c < c1) {
+      const uint4* src = trans + (static_cast<int64_t>(c) * p.H + h) * tr_step;
+      uint4* dst = ring + (c - c0) % kTransRing * tr_step;
+#pragma unroll
+      for (int i = 0; i < 2 * KS; ++i) attn::cp_async16(dst + i * 32, src + i * 32, true);
+    }
+    cp_async_commit();
+  };
+  copy(c0);
+  copy(c0 + 1);
+  fetch(c0);
   for (int c = c0; c < c1; ++c) {
     const int64_t ch = static_cast<int64_t>(c) * p.H + h;
     __nv_bfloat16* hi = buf + ((c - c0) & 1) * 2 * part;
@@ -442,7 +456,6 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
       *reinterpret_cast<uint32_t*>(hi + at + 8 * kPitch) = b.hi;
       *reinterpret_cast<uint32_t*>(lo + at + 8 * kPitch) = b.lo;
     }
-    uint4 th[kAhead ? KS : 1], tl[kAhead ? KS : 1];
     float acc[NT][4], lo1[NT][4], lo2[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
@@ -451,25 +464,13 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
       lo1[j][0] = lo1[j][1] = lo1[j][2] = lo1[j][3] = 0.f;
       lo2[j][0] = lo2[j][1] = lo2[j][2] = lo2[j][3] = 0.f;
     }
-    if constexpr (kAhead) {
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        th[ks] = nh[ks];
-        tl[ks] = nl[ks];
-      }
-    }
-    if (c + 1 < c1) fetch(c + 1);
+    fetch(c + 1);
+    cp_async_wait<kTransRing - 1>();
     __syncthreads();       // the other buffer is free as well: its readers have passed this barrier
+    const uint4* A = kRing ? ring + (c - c0) % kTransRing * tr_step : trans + ch * tr_step;
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
-      uint4 fh, fl;
-      if constexpr (kAhead) {
-        fh = th[ks];
-        fl = tl[ks];
-      } else {
-        fh = trans[ch * tr_step + ks * 64];
-        fl = trans[ch * tr_step + ks * 64 + 32];
-      }
+      const uint4 fh = A[ks * 64], fl = A[ks * 64 + 32];
       const uint32_t ah[4] = {fh.x, fh.y, fh.z, fh.w}, al[4] = {fl.x, fl.y, fl.z, fl.w};
       const int brow = (ks * 16 + (mat & 1) * 8 + mr) * kPitch + (mat >> 1) * 8;
 #pragma unroll
@@ -489,11 +490,13 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
         }
       }
     }
+    copy(c + kTransRing);
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = acc[j][e] + (lo1[j][e] + lo2[j][e]);
   }
+  cp_async_wait<0>();
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
     if (j >= tiles) break;
@@ -540,6 +543,16 @@ __global__ void __launch_bounds__(kThreads, TW <= 8 ? 2 : 1) delta_out_kernel(co
   };
   fetch(0);
   fetch(1);
+  // what the epilogue needs travels with the operands
+  const __nv_bfloat16* gate0 = reinterpret_cast<const __nv_bfloat16*>(p.z) + cp.t0 * p.ld + 2 * p.G * p.dk + p.H * p.dv + h * p.dv;
+  uint32_t gate[2][TW];
+#pragma unroll
+  for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+    for (int j = 0; j < TW; ++j) {
+      const int t = rb * 16 + rr * 8 + g;
+      gate[rr][j] = t < cp.n && j < tiles ? *reinterpret_cast<const uint32_t*>(gate0 + t * p.ld + (tile0 + j) * 8 + 2 * t4) : 0u;
+    }
   float acc[TW][4];
 #pragma unroll
   for (int j = 0; j < TW; ++j) {
@@ -590,7 +603,6 @@ __global__ void __launch_bounds__(kThreads, TW <= 8 ? 2 : 1) delta_out_kernel(co
     ssq[half][rb * 16 + g + 8] = q1;
   }
   __syncthreads();
-  const __nv_bfloat16* gate0 = reinterpret_cast<const __nv_bfloat16*>(p.z) + cp.t0 * p.ld + 2 * p.G * p.dk + p.H * p.dv + h * p.dv;
   __nv_bfloat16* out0 = reinterpret_cast<__nv_bfloat16*>(p.out) + cp.t0 * p.H * p.dv + h * p.dv;
 #pragma unroll
   for (int rr = 0; rr < 2; ++rr) {
@@ -601,9 +613,9 @@ __global__ void __launch_bounds__(kThreads, TW <= 8 ? 2 : 1) delta_out_kernel(co
     for (int j = 0; j < TW; ++j) {
       if (j >= tiles) break;
       const int c = (tile0 + j) * 8 + 2 * t4;
-      const float2 gt = ld2(gate0 + t * p.ld + c);
-      const float o0 = acc[j][2 * rr] * inv * p.norm_w[c] * gt.x * sigmoid_f32(gt.x);
-      const float o1 = acc[j][2 * rr + 1] * inv * p.norm_w[c + 1] * gt.y * sigmoid_f32(gt.y);
+      const float2 gt = unpack_bf16x2(gate[rr][j]);
+      const float o0 = acc[j][2 * rr] * inv * p.norm_w[c] * silu_f32(gt.x);
+      const float o1 = acc[j][2 * rr + 1] * inv * p.norm_w[c + 1] * silu_f32(gt.y);
       *reinterpret_cast<uint32_t*>(out0 + static_cast<int64_t>(t) * p.H * p.dv + c) = pack_bf16x2(o0, o1);
     }
   }
@@ -612,12 +624,12 @@ __global__ void __launch_bounds__(kThreads, TW <= 8 ? 2 : 1) delta_out_kernel(co
 template <int KS, int NT>
 cudaError_t launch_state(const DeltaArgs& a, cudaStream_t s) {
   static SmemOptIn opt;
-  constexpr int kMax = 2 * 2 * KS * 16 * (NT * 8 + 8) * 2;
-  cudaError_t e = opt.ensure(delta_state_kernel<KS, NT>, kMax);
+  constexpr size_t kSmem = state_smem<KS, NT>();
+  static_assert(kSmem <= 227 * 1024, "state pass must fit one SM");
+  cudaError_t e = opt.ensure(delta_state_kernel<KS, NT>, static_cast<int>(kSmem));
   if (e != cudaSuccess) return e;
   const int vtiles = a.dv / 8;
-  return launch_pdl(delta_state_kernel<KS, NT>, dim3((vtiles + NT - 1) / NT, a.H, a.N), dim3(a.dk * 2),
-                    static_cast<size_t>(2 * 2 * a.dk * (NT * 8 + 8) * 2), s, a);
+  return launch_pdl(delta_state_kernel<KS, NT>, dim3((vtiles + NT - 1) / NT, a.H, a.N), dim3(a.dk * 2), kSmem, s, a);
 }
 template <int NT>
 cudaError_t launch_state_nt(const DeltaArgs& a, cudaStream_t s) {
@@ -629,10 +641,13 @@ cudaError_t launch_state_nt(const DeltaArgs& a, cudaStream_t s) {
     case 5: return launch_state<5, NT>(a, s);
     case 6: return launch_state<6, NT>(a, s);
     case 8: return launch_state<8, NT>(a, s);
-    case 12: return launch_state<12, NT>(a, s);
-    case 16: return launch_state<16, NT>(a, s);
-    default: return cudaErrorInvalidValue;
+    default: break;
   }
+  if constexpr (NT <= 4) {
+    if (a.dk == 192) return launch_state<12, NT>(a, s);
+    if (a.dk == 256) return launch_state<16, NT>(a, s);
+  }
+  return cudaErrorInvalidValue;
 }
 template <int TW>
 cudaError_t launch_out(const DeltaArgs& a, cudaStream_t s) {
@@ -660,11 +675,14 @@ cudaError_t launch_delta_chunk(const DeltaArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   e = launch_pdl(delta_local_kernel, dim3(a.NC, a.H), dim3(kThreads), local_smem(a.dk), s, a);
   if (e != cudaSuccess) return e;
-  // every CTA of a head reads the same operands: narrow column tiles only while they still fit one wave
+  // every CTA of a head reads the same operands: narrower column tiles only while they still fit one wave
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  e = static_cast<int64_t>(a.N) * a.H * ((a.dv + 15) / 16) <= sms ? launch_state_nt<2>(a, s) : launch_state_nt<4>(a, s);
+  const int64_t heads = static_cast<int64_t>(a.N) * a.H;
+  e = heads * ((a.dv + 15) / 16) <= sms                   ? launch_state_nt<2>(a, s)
+      : heads * ((a.dv + 31) / 32) <= sms || a.dk > 128 ? launch_state_nt<4>(a, s)
+                                                          : launch_state_nt<8>(a, s);
   if (e != cudaSuccess) return e;
   if (a.dv <= 64) return launch_out<4>(a, s);
   if (a.dv <= 128) return launch_out<8>(a, s);

@@ -1,7 +1,7 @@
 // Latent attention on the 5th-generation tensor cores (bf16).
 //
 // latent_prefill_kernel   prompts, expanded form.  One CTA = 256 query rows of one head as two 128-row tiles that share every
-//                         block of 64 keys, as in the two-tile form of attn_sm100.cu (same softmax warps).  A key is
+//                         block of 64 keys, with the softmax warps of attn_sm100.cu's 128-row form.  A key is
 //                         [unrotated | rotated] from two tensors: the head's keys and the rotated part in the packed rows, which
 //                         all heads share; queries likewise.  Values arrive transposed from their GEMM.  Keys and values have
 //                         rings of their own: scores run a block ahead, so a key buffer is free a block earlier than the values
