@@ -144,8 +144,8 @@ __device__ bool splits_arrive_last(const DecodeParams& p) {
 }
 
 // Merge of the split partials of one head chunk by its last CTA: the partials come from other CTAs, so they are read
-// at L2.  First the LSEs of all heads of the chunk go to shared memory and become weights, then every thread sums four
-// output dims of one head over the splits with several independent 16-byte loads in flight and hands the normalised
+// at L2, in as few dependent round trips as it goes (it is the tail of a latency-bound kernel): a warp turns a head's LSEs into
+// weights, then every thread sums four output dims of one head over the splits with 16 loads in flight and hands the normalised
 // float4 to emit(head in chunk, b * Hq + head, float4 index, values, LSE of the head over all splits).
 template <int D, typename Emit>
 __device__ void merge_chunk(const DecodeParams& p, uint8_t* smem, Emit emit) {
@@ -156,47 +156,48 @@ __device__ void merge_chunk(const DecodeParams& p, uint8_t* smem, Emit emit) {
   float* s_w = reinterpret_cast<float*>(smem);          // [nheads][splits] weights
   float* s_inv = s_w + 16 * p.splits;                   // [nheads] 1 / total
   float* s_lse = s_inv + 16;                            // [nheads] LSE over all splits
-  for (int i = threadIdx.x; i < nheads * p.splits; i += kAttnThreads) {
-    const int h = i / p.splits, sp = i - h * p.splits;
-    s_w[i] = __ldcg(p.part_lse + (static_cast<int64_t>(b) * p.Hq + h_begin + h) * p.splits + sp);
-  }
-  __syncthreads();
-  if (threadIdx.x < nheads) {
-    float* w = s_w + threadIdx.x * p.splits;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int h = warp; h < nheads; h += kAttnThreads / 32) {      // a warp per head, a lane per split
+    const float* lse = p.part_lse + (static_cast<int64_t>(b) * p.Hq + h_begin + h) * p.splits;
+    float* w = s_w + h * p.splits;
     float mx = -INFINITY;
-    for (int i = 0; i < p.splits; ++i) mx = fmaxf(mx, w[i]);
+    for (int i = lane; i < p.splits; i += 32) {
+      w[i] = __ldcg(lse + i);
+      mx = fmaxf(mx, w[i]);
+    }
+    mx = warp_max(mx);
     float tot = 0.f;
-    for (int i = 0; i < p.splits; ++i) {
+    for (int i = lane; i < p.splits; i += 32) {
       const float e = (mx == -INFINITY) ? 0.f : __expf(w[i] - mx);
       w[i] = e;
       tot += e;
     }
-    s_inv[threadIdx.x] = tot > 0.f ? 1.f / tot : 0.f;
-    s_lse[threadIdx.x] = tot > 0.f ? mx + __logf(tot) : -INFINITY;
+    tot = warp_sum(tot);
+    if (lane == 0) {
+      s_inv[h] = tot > 0.f ? 1.f / tot : 0.f;
+      s_lse[h] = tot > 0.f ? mx + __logf(tot) : -INFINITY;
+    }
   }
   __syncthreads();
   constexpr int kVecPerHead = D / 4;                     // float4 per head row
   constexpr int kHeadsPerPass = kAttnThreads / kVecPerHead;
+  constexpr int kFlight = 16;                            // splits whose rows travel together
   const int dv = threadIdx.x % kVecPerHead, sub = threadIdx.x / kVecPerHead;
   for (int h = sub; h < nheads; h += kHeadsPerPass) {
     const int64_t bh = static_cast<int64_t>(b) * p.Hq + h_begin + h;
     const float4* po = reinterpret_cast<const float4*>(p.part_out + bh * p.splits * D) + dv;
     const float* w = s_w + h * p.splits;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    int i = 0;
-    for (; i + 8 <= p.splits; i += 8) {
-      float4 v[8];
+    for (int i = 0; i < p.splits; i += kFlight) {
+      float4 v[kFlight];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __ldcg(po + static_cast<int64_t>(i + j) * kVecPerHead);
+      for (int j = 0; j < kFlight; ++j)
+        v[j] = i + j < p.splits ? __ldcg(po + static_cast<int64_t>(i + j) * kVecPerHead) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc.x += w[i + j] * v[j].x; acc.y += w[i + j] * v[j].y;
-        acc.z += w[i + j] * v[j].z; acc.w += w[i + j] * v[j].w;
+      for (int j = 0; j < kFlight; ++j) {
+        const float f = i + j < p.splits ? w[i + j] : 0.f;
+        acc.x += f * v[j].x; acc.y += f * v[j].y; acc.z += f * v[j].z; acc.w += f * v[j].w;
       }
-    }
-    for (; i < p.splits; ++i) {
-      const float4 v = __ldcg(po + static_cast<int64_t>(i) * kVecPerHead);
-      acc.x += w[i] * v.x; acc.y += w[i] * v.y; acc.z += w[i] * v.z; acc.w += w[i] * v.w;
     }
     const float inv = s_inv[h];
     emit(h, bh, dv, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv), s_lse[h]);
