@@ -93,8 +93,8 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     """Prefill / context attention.  ``q`` [T, Hq, D] packed; query row i of sequence b has absolute position
     ``q_pos0[b] + i`` (default: the queries are the last ``q_len`` positions of the ``kv_lens[b]`` visible tokens).
 
-    ``impl``: "auto" picks the tcgen05 kernel (head dim 64 or 128, positive scale, at least ``SM100_PREFILL_MIN_Q`` query rows per
-    sequence) and otherwise the ``mma.sync`` kernel; "sm100" / "mma" force one.  ``max_kv_len`` (an upper bound of
+    ``impl``: "auto" picks the tcgen05 kernel (head dim 128, positive scale, at least ``SM100_PREFILL_MIN_Q`` query rows per
+    sequence; head dim 64 from ``SM100_PREFILL_MIN_Q_64`` rows on, with ``max_kv_len`` given and outside of a capture) and otherwise the ``mma.sync`` kernel; "sm100" / "mma" force one.  ``max_kv_len`` (an upper bound of
     ``kv_lens``) saves the tcgen05 path a device-to-host read.  ``softcap``: scores become ``softcap * tanh(score / softcap)``.
     ``sink`` fp32 [Hq]: exp(sink) joins every denominator (the LSE that is returned is that of the keys alone)."""
     D = q.shape[-1]
@@ -105,7 +105,10 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         sm100_ok = D in (64, 128) and scale > 0 and k_cache.dtype == torch.bfloat16 and os.environ.get("TDB200_ATTN_SM100", "1") != "0"
         if impl == "sm100" and not sm100_ok:
             raise ValueError("flash_attn_varlen: the tcgen05 kernel needs head dim 64 or 128, bf16 caches and a positive scale")
-        if impl == "sm100" or (impl == "auto" and sm100_ok and max_q_len >= (SM100_PREFILL_MIN_Q if D == 128 else SM100_PREFILL_MIN_Q_64)):
+        # heads of 64: not where the tcgen05 path would have to read a length or an error flag back (a capture must stay possible)
+        worth = max_q_len >= SM100_PREFILL_MIN_Q if D == 128 else (
+            max_q_len >= SM100_PREFILL_MIN_Q_64 and max_kv_len is not None and not torch.cuda.is_current_stream_capturing())
+        if impl == "sm100" or (impl == "auto" and sm100_ok and worth):
             if max_kv_len is None:
                 max_kv_len = int(kv_lens.max().item())
             out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous(),
