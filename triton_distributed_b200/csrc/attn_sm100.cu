@@ -322,7 +322,9 @@ __device__ __forceinline__ void softmax_duo(const FwdParams& p, uint64_t* s_full
   const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
   const uint32_t ts = tmem_s + lane_off;
   const int lim = (p.causal ? min(kv_len, pos0 + row0 + row + 1) : kv_len) - half * 64;   // tokens [0, lim) from this half's first are visible
-  constexpr float kRescaleStep = 8.f;            // log2, see softmax_tile
+  // log2, see softmax_tile.  Heads of 64 follow every new maximum, so that the largest probability stays an exact one in bf16 as in
+  // the mma.sync kernel that shorter prompts take
+  constexpr float kRescaleStep = D == 64 ? 0.f : 8.f;
   const float scale = CAP ? 1.f : p.scale_log2;
   float m = -INFINITY, l = 0.f;
   bool ok = true;
