@@ -109,6 +109,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, b
     return res
 
 
+@logged_op("gemm_swiglu", _gemm_meta)
 def gemm_swiglu(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``a`` [M, K], ``w`` [2 F, K] (gate rows, then up rows) -> ``silu(a gate^T) * (a up^T)`` [M, F].  From 256 rows on
     one launch of the CTA-pair kernel with the activation in its epilogue; fewer rows are a GEMM and an activation."""
