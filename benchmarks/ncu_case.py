@@ -3,6 +3,7 @@
   python benchmarks/ncu_case.py gemm      # tcgen05 GEMM 8192 x 4096 x 4096 (inputs + output ~160 MB > L2)
   python benchmarks/ncu_case.py skinny    # decode GEMM 32 x 5120 x 3200, split-K
   python benchmarks/ncu_case.py decode    # split-KV decode attention, 16 seqs x 4096 tokens, 8 q heads / 1 kv head
+  python benchmarks/ncu_case.py prompt    # causal prompt attention on tcgen05, 4096 tokens, 32 q heads / 8 kv heads of 128
   python benchmarks/ncu_case.py gemv      # decode GEMV 1 x 6400 x 5120 (65 MB of weights per launch, 4 weight copies)
   python benchmarks/ncu_case.py gemm_fp8  # block-scaled e4m3 GEMM 8192 x 3584 x 8192 (pair kernel, ~150 MB)
   python benchmarks/ncu_case.py moe       # grouped GEMM with in-kernel row gather: 8192 tokens, top-2 of 16 experts, 2048 x 2048
@@ -169,6 +170,13 @@ def main():
         lens = torch.full((B,), L, dtype=torch.int32, device="cuda")
         for _ in range(3):
             ops.gqa_fwd_batch_decode(q, k, v, None, None, lens, bt)
+    elif case == "prompt":
+        T = 4096
+        q = torch.randn(T, 32, 128, device="cuda", dtype=torch.bfloat16)
+        k, v = (torch.randn(1, T, 8, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        cu, lens = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, T], [T]))
+        for _ in range(3):
+            ops.flash_attn_varlen(q, k, v, ops.dense_block_table(1, "cuda"), cu, lens, T, max_kv_len=T)
     torch.cuda.synchronize()
     print("done", case)
 

@@ -71,7 +71,7 @@ def attention_reference(q, k_cache, v_cache, block_table, cu_seqlens_q, kv_lens,
 
 TENSOR_CORE_DIMS = (64, 128, 256)      # head dims of the mma.sync kernels (tcgen05: 64 and 128)
 SM100_PREFILL_MIN_Q = 128      # below this the 64-row mma.sync kernel has less padding and no KV packing pass
-SM100_PREFILL_MIN_Q_64 = 512   # heads of 64: 24 x 256 tokens 16.5 us against 12.4 of mma.sync, 512: 18.6 / 20.7, 8192: 323 / 1223
+SM100_PREFILL_MIN_Q_64 = 512   # heads of 64: 24 x 256 tokens 14.6 us against 10.5 of mma.sync, 512: 18.7 / 20.7, 8192: 342 / 1217
 _PENDING_ERRORS = []            # error flags of tcgen05 prefill launches that have not been looked at yet
 
 
