@@ -13,6 +13,7 @@ import torch
 
 from .. import _native
 from ..utils.oplog import logged_op
+from .elementwise import silu_mul
 
 
 SKINNY_M = 128   # up to this many rows the weight-streaming kernel wins
@@ -113,9 +114,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, b
 def gemm_swiglu(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``a`` [M, K], ``w`` [2 F, K] (gate rows, then up rows) -> ``silu(a gate^T) * (a up^T)`` [M, F].  From 256 rows on
     one launch of the CTA-pair kernel with the activation in its epilogue; fewer rows are a GEMM and an activation."""
-    from .elementwise import silu_mul
     M, N = a.numel() // a.shape[-1], w.shape[0]
-    if not (_native.use_native(a, w) and a.dtype == torch.bfloat16 and M >= 256 and N >= 512 and N % 16 == 0
+    if not (M >= 256 and N >= 512 and N % 16 == 0 and _native.use_native(a, w) and a.dtype == torch.bfloat16
             and a.stride(-1) == 1 and w.stride(-1) == 1 and os.environ.get("TDB200_GEMM_PAIR", "1") != "0"):
         return silu_mul(gemm(a, w))
     out = torch.empty((*a.shape[:-1], N // 2), dtype=a.dtype, device=a.device)
