@@ -173,6 +173,32 @@ def test_gated_group_gemm_and_sorted_rows(rt, T, E, k, H, I):
     assert act[:pad.numel()][pad].abs().max() == 0 if pad.any() else True
 
 
+@pytest.mark.parametrize("N,gated", [(320, False), (384, False), (448, False), (264, False), (384, True), (400, True)])
+def test_group_gemm_partial_column_tiles(rt, N, gated):
+    # widths that leave chunks of a tile's output without a store, several tiles per CTA and few products between the stores: a staging
+    # buffer must not be written again before its store has read it
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(N)
+    T, E, k, K = 148 * 128 * 2 + 5, 4, 2, 64
+    w = (torch.randn(E, N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    for _ in range(3):
+        x = torch.randn(T, K, device="cuda", dtype=torch.bfloat16)
+        ids = torch.rand(T, E, device="cuda").topk(k).indices.to(torch.int32)
+        srt = ops.sort_topk_ids_align_block_size(ids, E)
+        y = ops.group_gemm_gather(x, w, srt, a_row_div=k, gated=gated)[srt.pos_of.long()].double()
+        torch.cuda.synchronize()
+        pairs, rows = ids.reshape(-1), x.repeat_interleave(k, 0)
+        for e in range(E):
+            at = pairs == e
+            ref = rows[at].double() @ w[e].double().t()
+            if gated:
+                g, u = ref.chunk(2, -1)
+                ref = torch.nn.functional.silu(g) * u
+            # one rounding to bf16 of values of order one, and fp32 sums
+            torch.testing.assert_close(y[at], ref, rtol=2 ** -8, atol=2 ** -10)
+
+
 @pytest.mark.parametrize("E", [1, 31, 128, 129, 512])
 def test_router_bf16_logits(E):
     from triton_distributed_b200.ops import topk_router

@@ -604,9 +604,9 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
           if (p.tma_y) {
             fence_proxy_async_smem();
             epi_bar();
-            if (leader && col0 < width) {
-              tma_store_2d(&tmap_y, stg, col0, mt * kBM);
-              bulk_commit();
+            if (leader) {
+              if (col0 < width) tma_store_2d(&tmap_y, stg, col0, mt * kBM);
+              bulk_commit();      // a group per chunk, empty past the last column: the wait above counts groups
             }
           }
         }
