@@ -214,6 +214,29 @@ def test_gemm_swiglu(M, F, K):
     torch.testing.assert_close(out.double(), ref, rtol=2 ** -8 if M >= 256 else 2 ** -6, atol=2 ** -10 if M >= 256 else 2 ** -8)
 
 
+@pytest.mark.parametrize("form", ["pair", "gated", "single"])
+@pytest.mark.parametrize("M,N", [(256 * 148 + 9, 320), (256 * 148 + 9, 528), (256 * 148 + 137, 768), (128 * 444, 392)])
+def test_gemm_chunks_without_a_store(M, N, form):
+    # columns and rows that leave chunks of a tile without a store, several tiles per CTA and few products between the stores: a staging
+    # buffer must not be written again before its store has read it
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(N)
+    K = 64
+    if form == "gated":
+        N *= 2
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    for _ in range(3):
+        x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+        out = ops.gemm_swiglu(x, w) if form == "gated" else ops.gemm(x, w, block_n=512 if form == "pair" else 256)
+        ref = x.double() @ w.double().t()
+        if form == "gated":
+            g, u = ref.chunk(2, dim=-1)
+            ref = torch.nn.functional.silu(g) * u
+        # one rounding to bf16 of values of order one behind fp32 sums
+        torch.testing.assert_close(out.double(), ref, rtol=2 ** -8, atol=2 ** -10)
+
+
 @pytest.mark.parametrize("M,F,K", [(1, 4, 8), (1, 3, 264), (2, 1001, 520), (4, 12288, 256), (7, 149, 2048), (16, 300, 4096), (1, 70, 40000)])
 def test_gemv_swiglu(M, F, K):
     # groups of four gate and four up rows: whole, shared by warps, partly empty

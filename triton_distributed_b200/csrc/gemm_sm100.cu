@@ -700,9 +700,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             }
             fence_proxy_async_smem();
             epi_bar();
-            if (leader && tl.n0 + c * kEpiCols < p.N) {
-              tma_store_3d(cmap, stg, tl.n0 + c * kEpiCols, tl.mt * kBM, c2);
-              bulk_commit();
+            if (leader) {
+              if (tl.n0 + c * kEpiCols < p.N) tma_store_3d(cmap, stg, tl.n0 + c * kEpiCols, tl.mt * kBM, c2);
+              bulk_commit();      // a group per chunk, empty past the last column: the wait above counts groups
             }
           }
           if (p.mode == kGemmReduceScatter && leader) {
@@ -1166,9 +1166,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           fence_proxy_async_smem();
           epi_bar();
-          if (leader && valid_m && tl.n0 / 2 + c * kEpiCols < p.N / 2) {
-            tma_store_3d(&tmap_c, stg, tl.n0 / 2 + c * kEpiCols, mt * kBM, tl.seg);
-            bulk_commit();
+          if (leader) {
+            if (valid_m && tl.n0 / 2 + c * kEpiCols < p.N / 2) tma_store_3d(&tmap_c, stg, tl.n0 / 2 + c * kEpiCols, mt * kBM, tl.seg);
+            bulk_commit();        // a group per chunk, empty where nothing is stored: the wait above counts groups
           }
         }
 #pragma unroll 1
@@ -1250,9 +1250,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           fence_proxy_async_smem();
           epi_bar();
-          if (leader && valid_m && tl.n0 + c * kEpiCols < p.N) {
-            tma_store_3d(cmap, stg, tl.n0 + c * kEpiCols, mt * kBM, c2);
-            bulk_commit();
+          if (leader) {
+            if (valid_m && tl.n0 + c * kEpiCols < p.N) tma_store_3d(cmap, stg, tl.n0 + c * kEpiCols, mt * kBM, c2);
+            bulk_commit();        // as in the gated loop
           }
         }
         if (p.mode == kGemmReduceScatter && !own_seg && leader && valid_m) {
