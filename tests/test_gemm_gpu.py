@@ -198,6 +198,23 @@ def test_gemv_spans(M, N, K):
     assert ((out - ref).abs() <= ref.abs() * 2 ** -8 + 2 ** -20 * K ** 0.5 + 1e-5).all()
 
 
+@pytest.mark.parametrize("M", [1, 3, 8, 16])
+def test_gemv_empty_sums(M):
+    # no input features: the residual alone, or zeros, whatever the prologue; no output features: nothing to do
+    from triton_distributed_b200 import ops
+
+    x = torch.randn(M, 64, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(304, 64, device="cuda", dtype=torch.bfloat16)
+    res = torch.randn(M, 304, device="cuda", dtype=torch.bfloat16)
+    none = torch.ones(0, device="cuda", dtype=torch.bfloat16)
+    for kw, want in ((dict(), torch.zeros_like(res)), (dict(residual=res), res), (dict(norm_weight=none), torch.zeros_like(res)),
+                     (dict(silu_mul=True, residual=res), res), (dict(swiglu=True), torch.zeros_like(res[:, :152]))):
+        out = ops.gemv_fused(x[:, :0], w[:, :0], out=torch.full_like(want, 7.0), **kw)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want), kw
+        assert ops.gemv_fused(x, w[:0], **{k: v for k, v in kw.items() if k == "swiglu"}).shape == (M, 0)
+
+
 @pytest.mark.parametrize("M,F,K", [(256, 256, 64), (257, 264, 200), (777, 520, 1024), (1024, 19 * 128, 128), (300, 5000, 72), (8, 384, 512)])
 def test_gemm_swiglu(M, F, K):
     # gate and up columns that end inside a tile's halves, half-width tail tiles, rows that end inside a CTA's 128; few rows: two launches
