@@ -69,3 +69,20 @@ def test_gdn_chunk_kernels_over_column_tiles_and_sequence_ends(H, V, lens):
     assert (ht - s_r).norm().item() < 2 ** -7 * s_r.norm().item()
     empty = [i for i, n in enumerate(lens) if n == 0]
     assert torch.equal(ht[empty], h0[empty])
+
+
+def test_gdn_state_at_an_odd_address():
+    """A contiguous initial state may begin at any element of its storage."""
+    from test_gdn_cpu import _inputs
+    from triton_distributed_b200 import ops
+
+    H, K, V, lens = 2, 128, 64, [70, 5]
+    cu = torch.tensor([0, 70, 75], dtype=torch.int32, device="cuda")
+    q, k, v, g, beta = _inputs(75, H, K, V, seed=4, dtype=torch.bfloat16, device="cuda")
+    flat = torch.randn(len(lens) * H * K * V + 3, device="cuda") * 0.1
+    for first in (1, 2, 3):
+        h0 = flat[first:first + len(lens) * H * K * V].view(len(lens), H, K, V)
+        got = ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, h0, True, cu, impl="chunk")
+        want = ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, h0.clone(), True, cu, impl="chunk")
+        torch.cuda.synchronize()
+        assert torch.equal(got[1], want[1]) and torch.equal(got[3], want[3])

@@ -277,7 +277,7 @@ std::tuple<at::Tensor, at::Tensor> gdn_fwd(const at::Tensor& q, const at::Tensor
   return {o, ht};
 }
 
-// Chunk-parallel gated delta rule forward.  chunk_seq / chunk_t0 int32 [NC], seq_chunk0 int32 [N + 1] (device).
+// Chunk-parallel gated delta rule forward.
 // Returns (o bf16 [T, H, V], g_cumsum fp32 [T, H], A fp32 [T, H, 64] or empty, final_state fp32 [N, H, K, V] or empty).
 std::vector<at::Tensor> gdn_chunk_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g,
                                       const at::Tensor& beta, double scale, const c10::optional<at::Tensor>& h0,
@@ -318,10 +318,13 @@ std::vector<at::Tensor> gdn_chunk_fwd(const at::Tensor& q, const at::Tensor& k, 
   a.a_out = return_a ? A.data_ptr<float>() : nullptr;
   a.w = w.data_ptr(); a.kd = kd.data_ptr(); a.u = u.data_ptr(); a.v_new = vn.data_ptr(); a.h_chunks = hs.data_ptr();
   a.initial_state = nullptr;
+  at::Tensor h0_aligned;
   if (h0.has_value()) {
     TORCH_CHECK(h0->scalar_type() == at::kFloat && h0->is_contiguous() && h0->numel() == N * H * K * V,
                 "gdn_chunk_fwd: initial_state fp32 [N, H, K, V]");
-    a.initial_state = h0->data_ptr<float>();
+    // the state walk reads pairs of floats
+    if (reinterpret_cast<uintptr_t>(h0->data_ptr()) % 8 != 0) h0_aligned = h0->clone();
+    a.initial_state = h0_aligned.defined() ? h0_aligned.data_ptr<float>() : h0->data_ptr<float>();
   }
   a.final_state = output_final_state ? ht.data_ptr<float>() : nullptr;
   a.o = o.data_ptr();
