@@ -149,3 +149,28 @@ def test_prefill_two_tiles(D, qlens, kvlens, pos0, cap, sink, causal):
     seen = ref_lse > float("-inf")
     assert torch.equal(lse > float("-inf"), seen)
     torch.testing.assert_close(lse[seen], ref_lse[seen], rtol=1e-4, atol=1e-4)
+
+
+def _prompts_of_64(first=0, T=600, Hq=4, Hkv=2, lens=(600, 900), page=40):
+    # two prompts of heads of 64, long enough for the tcgen05 kernel; q begins at element ``first`` of its storage
+    B, D = len(lens), 64
+    k, v, bt = _paged_cache(B, max(lens), Hkv, D, page, seed=7)
+    q = torch.randn(B * T * Hq * D + 8, device="cuda").to(torch.bfloat16)[first:first + B * T * Hq * D].view(B * T, Hq, D)
+    cu = torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device="cuda")
+    return q, k, v, bt, cu, torch.tensor(lens, dtype=torch.int32, device="cuda"), T
+
+
+@pytest.mark.parametrize("first,cap", [(2, 0.0), (4, 0.0), (6, 5.0), (0, -3.0)])
+def test_prefill_heads_of_64_what_tma_cannot_take(first, cap):
+    from triton_distributed_b200.ops import flash_attn_varlen
+
+    args = _prompts_of_64(first)
+    out = flash_attn_varlen(*args, softcap=cap, max_kv_len=900)
+    want = flash_attn_varlen(*args, softcap=cap, max_kv_len=900, impl="mma")
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    q, k, v, bt, cu, lens, T = args
+    wide = torch.stack([bt, bt], 1)[:, 0]
+    for impl in ("auto", "mma"):
+        with pytest.raises(RuntimeError, match="block_table"):
+            flash_attn_varlen(q, k, v, wide, cu, lens, T, max_kv_len=900, impl=impl)

@@ -105,15 +105,18 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         sm100_ok = D in (64, 128) and scale > 0 and k_cache.dtype == torch.bfloat16 and os.environ.get("TDB200_ATTN_SM100", "1") != "0"
         if impl == "sm100" and not sm100_ok:
             raise ValueError("flash_attn_varlen: the tcgen05 kernel needs head dim 64 or 128, bf16 caches and a positive scale")
-        # heads of 64: not where the tcgen05 path would have to read a length or an error flag back (a capture must stay possible)
+        # heads of 64: not where the tcgen05 path would have to read a length or an error flag back (a capture must stay possible), nor
+        # with a negative soft cap (none to the mma.sync kernel) or a q that TMA cannot address
         worth = max_q_len >= SM100_PREFILL_MIN_Q if D == 128 else (
-            max_q_len >= SM100_PREFILL_MIN_Q_64 and max_kv_len is not None and not torch.cuda.is_current_stream_capturing())
+            max_q_len >= SM100_PREFILL_MIN_Q_64 and max_kv_len is not None and softcap >= 0 and (q.data_ptr() % 16 == 0 or not q.is_contiguous())
+            and not torch.cuda.is_current_stream_capturing())
         if impl == "sm100" or (impl == "auto" and sm100_ok and worth):
             if max_kv_len is None:
                 max_kv_len = int(kv_lens.max().item())
-            out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous(),
-                                           cu_seqlens_q, kv_lens, q_pos0, int(max_q_len), max(int(max_kv_len), 1),
-                                           bool(causal), float(scale), lse, None, sink, None, float(softcap))
+            if D == 128:      # heads of 64 refuse what the mma.sync kernel refuses
+                k_cache, v_cache, block_table = k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous()
+            out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache, v_cache, block_table, cu_seqlens_q, kv_lens, q_pos0, int(max_q_len),
+                                           max(int(max_kv_len), 1), bool(causal), float(scale), lse, None, sink, None, float(softcap))
             _PENDING_ERRORS.append(err)
             if len(_PENDING_ERRORS) > 64:
                 check_attention_errors()
