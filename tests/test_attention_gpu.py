@@ -174,3 +174,38 @@ def test_prefill_heads_of_64_what_tma_cannot_take(first, cap):
     for impl in ("auto", "mma"):
         with pytest.raises(RuntimeError, match="block_table"):
             flash_attn_varlen(q, k, v, wide, cu, lens, T, max_kv_len=900, impl=impl)
+
+
+@pytest.mark.parametrize("page", [40, 900])
+def test_prefill_heads_of_64_do_not_depend_on_a_length_bound(page):
+    # the block table says how many positions there may be; max_kv_len never mattered to these heads
+    from triton_distributed_b200.ops import attention_reference, flash_attn_varlen
+
+    q, k, v, bt, cu, lens, T = _prompts_of_64(page=page)
+    ref = attention_reference(q.float(), k.float(), v.float(), bt, cu, lens)
+    outs = [flash_attn_varlen(q, k, v, bt, cu, lens, T, max_kv_len=n) for n in (1, 64, 640, 900, 5000)]
+    torch.cuda.synchronize()
+    # probabilities and output are rounded to bf16, 2^-9 each, in sums of values of order one
+    torch.testing.assert_close(outs[0].float(), ref.float(), rtol=2 ** -7, atol=2 ** -6)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+def test_prefill_heads_of_64_without_room_for_scratch(monkeypatch):
+    # more scratch than the limit, or none to be had: the kernel that needs none
+    from triton_distributed_b200.ops import attention, flash_attn_varlen
+
+    args = _prompts_of_64()
+    want = flash_attn_varlen(*args, max_kv_len=900, impl="mma")
+    monkeypatch.setattr(attention, "SM100_SCRATCH_64", 2 * 2 * 2 * 960 * 64 * 2 - 1)
+    assert torch.equal(flash_attn_varlen(*args, max_kv_len=900), want)
+    monkeypatch.undo()
+    tcgen05 = flash_attn_varlen(*args, max_kv_len=900)
+
+    def full(*a, **kw):
+        raise torch.cuda.OutOfMemoryError("no memory left")
+
+    monkeypatch.setattr(attention.torch, "empty", full)
+    got = flash_attn_varlen(*args, max_kv_len=900)
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and not torch.equal(tcgen05, want)

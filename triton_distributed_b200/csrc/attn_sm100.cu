@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(256) attn_pack_kv_kernel(const PackParams p) {
   __shared__ __align__(16) __nv_bfloat16 vs[kBN][D + 8];
   const int t0 = blockIdx.x * kBN, h = blockIdx.y, b = blockIdx.z;
   const int kv_len = p.kv_lens[b];
+  if (t0 >= (kv_len + 127) / 128 * 128) return;      // no block of 64 or 128 keys reaches that far
   const int64_t bh = static_cast<int64_t>(b) * p.Hkv + h;
   for (int i = threadIdx.x; i < kBN * (D / 8); i += 256) {
     const int r = i / (D / 8), c = (i % (D / 8)) * 8;

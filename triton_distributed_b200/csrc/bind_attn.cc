@@ -102,13 +102,14 @@ at::Tensor flash_fwd(const at::Tensor& q, const at::Tensor& k_cache, const at::T
   return out;
 }
 
-// Prefill attention on the tcgen05 path (head dim 128).  Returns (out, error flag int32[1]: non-zero if a bounded wait
-// inside the kernel gave up).
+// Prefill attention on the tcgen05 path (head dim 64 or 128).  Returns (out, error flag int32[1]: non-zero if a bounded wait
+// inside the kernel gave up).  scratch: room for the dense K and V^T, bf16 (allocated here without it).
 std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
                                         const at::Tensor& block_table, const at::Tensor& cu_seqlens_q, const at::Tensor& kv_lens,
                                         c10::optional<at::Tensor> q_pos0, int64_t max_q_len, int64_t max_kv_len, bool causal,
                                         double scale, c10::optional<at::Tensor> lse, c10::optional<at::Tensor> k_scale,
-                                        c10::optional<at::Tensor> sink, c10::optional<at::Tensor> gate, double softcap) {
+                                        c10::optional<at::Tensor> sink, c10::optional<at::Tensor> gate, double softcap,
+                                        c10::optional<at::Tensor> scratch) {
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.scalar_type() == at::kBFloat16 && (q.size(2) == 128 || q.size(2) == 64),
               "flash_fwd_sm100: q must be contiguous bf16 [T, Hq, 64 or 128]");
   TORCH_CHECK(k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.is_contiguous() &&
@@ -148,10 +149,12 @@ std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k
   a.softcap = softcap;
   TORCH_CHECK(max_kv_len >= 1, "flash_fwd_sm100: max_kv_len must be positive");
   a.Lp = static_cast<int>((max_kv_len + 63) / 64 * 64);
-  at::Tensor kd = at::empty({a.batch * a.num_kv_heads, a.Lp, a.head_dim}, q.options());
-  at::Tensor vt = at::empty({a.batch * a.num_kv_heads, a.head_dim, a.Lp}, q.options());
-  a.k_dense = kd.data_ptr();
-  a.vt_dense = vt.data_ptr();
+  const int64_t half = static_cast<int64_t>(a.batch) * a.num_kv_heads * a.Lp * a.head_dim;
+  at::Tensor dense = scratch.has_value() ? *scratch : at::empty({2 * half}, q.options());
+  TORCH_CHECK(dense.scalar_type() == at::kBFloat16 && dense.is_cuda() && dense.is_contiguous() && dense.numel() >= 2 * half,
+              "flash_fwd_sm100: scratch too small");
+  a.k_dense = dense.data_ptr();
+  a.vt_dense = dense.data_ptr<at::BFloat16>() + half;
   a.error_flag = err.data_ptr<int32_t>();
   set_k_scale(a.kv, k_cache, k_scale);
   a.epi = make_epilogue(q, sink, gate);
@@ -301,7 +304,7 @@ void bind_attn(py::module_& m) {
   m.def("flash_fwd_sm100", &flash_fwd_sm100, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("cu_seqlens_q"), py::arg("kv_lens"), py::arg("q_pos0"), py::arg("max_q_len"), py::arg("max_kv_len"),
         py::arg("causal"), py::arg("scale"), py::arg("lse"), py::arg("k_scale") = py::none(), py::arg("sink") = py::none(),
-        py::arg("gate") = py::none(), py::arg("softcap") = 0.0);
+        py::arg("gate") = py::none(), py::arg("softcap") = 0.0, py::arg("scratch") = py::none());
   m.def("decode_attn", &decode_attn, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("kv_lens"), py::arg("workspace"), py::arg("splits"), py::arg("scale"), py::arg("softcap"), py::arg("out"),
         py::arg("out_lse"), py::arg("out_f32"), py::arg("counters"), py::arg("k_scale") = py::none(),

@@ -72,6 +72,7 @@ def attention_reference(q, k_cache, v_cache, block_table, cu_seqlens_q, kv_lens,
 TENSOR_CORE_DIMS = (64, 128, 256)      # head dims of the mma.sync kernels (tcgen05: 64 and 128)
 SM100_PREFILL_MIN_Q = 128      # below this the 64-row mma.sync kernel has less padding and no KV packing pass
 SM100_PREFILL_MIN_Q_64 = 512   # heads of 64: 24 x 256 tokens 14.6 us against 10.5 of mma.sync, 512: 18.7 / 20.7, 8192: 342 / 1217
+SM100_SCRATCH_64 = 256 << 20   # heads of 64: most bytes of scratch (8 sequences x 4 heads x 32768 positions)
 _PENDING_ERRORS = []            # error flags of tcgen05 prefill launches that have not been looked at yet
 
 
@@ -85,6 +86,22 @@ def check_attention_errors() -> None:
         raise RuntimeError("flash_fwd_sm100: a wait inside the kernel timed out")
 
 
+def _scratch_64(kv_lens: torch.Tensor, k_cache: torch.Tensor, block_table: torch.Tensor, limit: Optional[int]):
+    """(positions, scratch) of the tcgen05 kernel for heads of 64: dense K and V^T of every position that the block table can name, so
+    that nothing depends on a caller's ``max_kv_len``, which the mma.sync kernel does not look at.  No scratch (None) beyond ``limit``
+    bytes or where there is no memory left for it."""
+    positions = max(block_table.shape[1] * k_cache.shape[1], 1)
+    elements = 2 * kv_lens.numel() * k_cache.shape[2] * ((positions + 63) // 64 * 64) * 64
+    if limit is not None and 2 * elements > limit:
+        return positions, None
+    try:
+        return positions, torch.empty(elements, dtype=k_cache.dtype, device=k_cache.device)
+    except torch.cuda.OutOfMemoryError:
+        if limit is None:
+            raise
+        return positions, None
+
+
 def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                       cu_seqlens_q: torch.Tensor, kv_lens: torch.Tensor, max_q_len: int,
                       q_pos0: Optional[torch.Tensor] = None, causal: bool = True, scale: Optional[float] = None,
@@ -94,8 +111,9 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     ``q_pos0[b] + i`` (default: the queries are the last ``q_len`` positions of the ``kv_lens[b]`` visible tokens).
 
     ``impl``: "auto" picks the tcgen05 kernel (head dim 128, positive scale, at least ``SM100_PREFILL_MIN_Q`` query rows per
-    sequence; head dim 64 from ``SM100_PREFILL_MIN_Q_64`` rows on, with ``max_kv_len`` given and outside of a capture) and otherwise the ``mma.sync`` kernel; "sm100" / "mma" force one.  ``max_kv_len`` (an upper bound of
-    ``kv_lens``) saves the tcgen05 path a device-to-host read.  ``softcap``: scores become ``softcap * tanh(score / softcap)``.
+    sequence; head dim 64 from ``SM100_PREFILL_MIN_Q_64`` rows on, with ``max_kv_len`` given, outside of a capture and with at most
+    ``SM100_SCRATCH_64`` bytes of scratch) and otherwise the ``mma.sync`` kernel; "sm100" / "mma" force one.  ``max_kv_len`` (an
+    upper bound of ``kv_lens``) saves the tcgen05 path a device-to-host read.  ``softcap``: scores become ``softcap * tanh(score / softcap)``.
     ``sink`` fp32 [Hq]: exp(sink) joins every denominator (the LSE that is returned is that of the keys alone)."""
     D = q.shape[-1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
@@ -110,13 +128,17 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         worth = max_q_len >= SM100_PREFILL_MIN_Q if D == 128 else (
             max_q_len >= SM100_PREFILL_MIN_Q_64 and max_kv_len is not None and softcap >= 0 and (q.data_ptr() % 16 == 0 or not q.is_contiguous())
             and not torch.cuda.is_current_stream_capturing())
+        scratch = None
+        if D == 64 and (impl == "sm100" or (impl == "auto" and sm100_ok and worth)):
+            max_kv_len, scratch = _scratch_64(kv_lens, k_cache, block_table, SM100_SCRATCH_64 if impl == "auto" else None)
+            worth = scratch is not None
         if impl == "sm100" or (impl == "auto" and sm100_ok and worth):
             if max_kv_len is None:
                 max_kv_len = int(kv_lens.max().item())
             if D == 128:      # heads of 64 refuse what the mma.sync kernel refuses
                 k_cache, v_cache, block_table = k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous()
             out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache, v_cache, block_table, cu_seqlens_q, kv_lens, q_pos0, int(max_q_len),
-                                           max(int(max_kv_len), 1), bool(causal), float(scale), lse, None, sink, None, float(softcap))
+                                           max(int(max_kv_len), 1), bool(causal), float(scale), lse, None, sink, None, float(softcap), scratch)
             _PENDING_ERRORS.append(err)
             if len(_PENDING_ERRORS) > 64:
                 check_attention_errors()
