@@ -209,3 +209,29 @@ def test_prefill_heads_of_64_without_room_for_scratch(monkeypatch):
     monkeypatch.undo()
     torch.cuda.synchronize()
     assert torch.equal(got, want) and not torch.equal(tcgen05, want)
+
+
+def test_prefill_heads_of_64_wait_for_nothing():
+    # however many calls: no error flag is read back
+    from triton_distributed_b200.ops import attention, flash_attn_varlen
+
+    args = _prompts_of_64()
+    flash_attn_varlen(*args, max_kv_len=900)
+    attention.check_attention_errors()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        for _ in range(150):
+            flash_attn_varlen(*args, max_kv_len=900)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    assert not attention._PENDING_ERRORS
+    # what a kernel reports is raised by the next call, once
+    torch.cuda.synchronize()
+    attention._STATUS_WORDS["word"][0] = 1
+    with pytest.raises(RuntimeError, match="timed out"):
+        flash_attn_varlen(*args, max_kv_len=900)
+    flash_attn_varlen(*args, max_kv_len=900)
+    attention._STATUS_WORDS["word"][0] = 2
+    with pytest.raises(RuntimeError, match="aligned"):
+        attention.check_attention_errors()
+    attention.check_attention_errors()

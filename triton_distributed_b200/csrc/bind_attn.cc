@@ -103,13 +103,14 @@ at::Tensor flash_fwd(const at::Tensor& q, const at::Tensor& k_cache, const at::T
 }
 
 // Prefill attention on the tcgen05 path (head dim 64 or 128).  Returns (out, error flag int32[1]: non-zero if a bounded wait
-// inside the kernel gave up).  scratch: room for the dense K and V^T, bf16 (allocated here without it).
+// inside the kernel gave up).  scratch: room for the dense K and V^T, bf16 (allocated here without it).  status: the flag to use, in
+// pinned host memory (a new one on the device without it).
 std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k_cache, const at::Tensor& v_cache,
                                         const at::Tensor& block_table, const at::Tensor& cu_seqlens_q, const at::Tensor& kv_lens,
                                         c10::optional<at::Tensor> q_pos0, int64_t max_q_len, int64_t max_kv_len, bool causal,
                                         double scale, c10::optional<at::Tensor> lse, c10::optional<at::Tensor> k_scale,
                                         c10::optional<at::Tensor> sink, c10::optional<at::Tensor> gate, double softcap,
-                                        c10::optional<at::Tensor> scratch) {
+                                        c10::optional<at::Tensor> scratch, c10::optional<at::Tensor> status) {
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && q.scalar_type() == at::kBFloat16 && (q.size(2) == 128 || q.size(2) == 64),
               "flash_fwd_sm100: q must be contiguous bf16 [T, Hq, 64 or 128]");
   TORCH_CHECK(k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.is_contiguous() &&
@@ -121,7 +122,7 @@ std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k
   c10::cuda::CUDAGuard guard(q.device());
   tdb::FlashFwdSm100Args a;
   at::Tensor out = at::empty_like(q);
-  at::Tensor err = at::zeros({1}, q.options().dtype(at::kInt));
+  at::Tensor err = status.has_value() ? *status : at::zeros({1}, q.options().dtype(at::kInt));
   a.q = q.data_ptr();
   a.out = out.data_ptr();
   a.lse = nullptr;
@@ -156,6 +157,10 @@ std::vector<at::Tensor> flash_fwd_sm100(const at::Tensor& q, const at::Tensor& k
   a.k_dense = dense.data_ptr();
   a.vt_dense = dense.data_ptr<at::BFloat16>() + half;
   a.error_flag = err.data_ptr<int32_t>();
+  if (status.has_value()) {
+    TORCH_CHECK(err.is_cpu() && err.numel() == 1, "flash_fwd_sm100: status must be one word of pinned host memory");
+    check_cuda(cudaHostGetDevicePointer(reinterpret_cast<void**>(&a.error_flag), err.data_ptr(), 0), "status word");
+  }
   set_k_scale(a.kv, k_cache, k_scale);
   a.epi = make_epilogue(q, sink, gate);
   check_cuda(tdb::launch_flash_fwd_sm100(a, cur_stream()), "launch_flash_fwd_sm100");
@@ -304,7 +309,8 @@ void bind_attn(py::module_& m) {
   m.def("flash_fwd_sm100", &flash_fwd_sm100, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("cu_seqlens_q"), py::arg("kv_lens"), py::arg("q_pos0"), py::arg("max_q_len"), py::arg("max_kv_len"),
         py::arg("causal"), py::arg("scale"), py::arg("lse"), py::arg("k_scale") = py::none(), py::arg("sink") = py::none(),
-        py::arg("gate") = py::none(), py::arg("softcap") = 0.0, py::arg("scratch") = py::none());
+        py::arg("gate") = py::none(), py::arg("softcap") = 0.0, py::arg("scratch") = py::none(),
+        py::arg("status") = py::none());
   m.def("decode_attn", &decode_attn, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"),
         py::arg("kv_lens"), py::arg("workspace"), py::arg("splits"), py::arg("scale"), py::arg("softcap"), py::arg("out"),
         py::arg("out_lse"), py::arg("out_f32"), py::arg("counters"), py::arg("k_scale") = py::none(),

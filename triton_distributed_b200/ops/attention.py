@@ -74,12 +74,32 @@ SM100_PREFILL_MIN_Q = 128      # below this the 64-row mma.sync kernel has less 
 SM100_PREFILL_MIN_Q_64 = 512   # heads of 64: 24 x 256 tokens 14.6 us against 10.5 of mma.sync, 512: 18.7 / 20.7, 8192: 342 / 1217
 SM100_SCRATCH_64 = 256 << 20   # heads of 64: most bytes of scratch (8 sequences x 4 heads x 32768 positions)
 _PENDING_ERRORS = []            # error flags of tcgen05 prefill launches that have not been looked at yet
+_STATUS_WORDS = {}              # "word": the error flag of launches whose callers never waited for the device, in pinned host memory
+
+
+def _status_word() -> torch.Tensor:
+    """The word that tcgen05 launches of heads of 64 report to.  It is looked at here, before every such launch, without a wait: an
+    error shows at the first call behind it, or in :func:`check_attention_errors`."""
+    word = _STATUS_WORDS.get("word")
+    if word is None:
+        word = _STATUS_WORDS.setdefault("word", torch.zeros(1, dtype=torch.int32).pin_memory())
+    _raise_for([int(word.numpy()[0])])
+    return word
 
 
 def check_attention_errors() -> None:
     """Raise if a bounded wait inside a tcgen05 prefill kernel gave up since the last check (synchronises)."""
     flags, _PENDING_ERRORS[:] = list(_PENDING_ERRORS), []
     codes = [int(f.item()) for f in flags]
+    if "word" in _STATUS_WORDS:
+        torch.cuda.synchronize()
+        codes.append(int(_STATUS_WORDS["word"].numpy()[0]))
+    _raise_for(codes)
+
+
+def _raise_for(codes) -> None:
+    if any(codes) and "word" in _STATUS_WORDS:
+        _STATUS_WORDS["word"].zero_()
     if any(c == 2 for c in codes):
         raise RuntimeError("flash_fwd_sm100: the dynamic shared-memory window was not 1024-byte aligned")
     if any(c != 0 for c in codes):
@@ -138,10 +158,12 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
             if D == 128:      # heads of 64 refuse what the mma.sync kernel refuses
                 k_cache, v_cache, block_table = k_cache.contiguous(), v_cache.contiguous(), block_table.contiguous()
             out, err = lib.flash_fwd_sm100(q.contiguous(), k_cache, v_cache, block_table, cu_seqlens_q, kv_lens, q_pos0, int(max_q_len),
-                                           max(int(max_kv_len), 1), bool(causal), float(scale), lse, None, sink, None, float(softcap), scratch)
-            _PENDING_ERRORS.append(err)
-            if len(_PENDING_ERRORS) > 64:
-                check_attention_errors()
+                                           max(int(max_kv_len), 1), bool(causal), float(scale), lse, None, sink, None, float(softcap), scratch,
+                                           _status_word() if D == 64 else None)
+            if D == 128:
+                _PENDING_ERRORS.append(err)
+                if len(_PENDING_ERRORS) > 64:
+                    check_attention_errors()
             return (out, lse) if return_lse else out
         out = lib.flash_fwd(q.contiguous(), k_cache, v_cache, block_table, cu_seqlens_q, kv_lens, q_pos0, int(max_q_len),
                             bool(causal), float(scale), float(softcap), lse, None, sink)
