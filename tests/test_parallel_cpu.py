@@ -124,3 +124,16 @@ def _pp(rank, world):
 
 def test_pp_transport_two_ranks():
     run_cpu_ranks(_pp, 2)
+
+
+def test_flash_decode_shard_splits_and_launch_form():
+    # batch x KV heads fixes how far a shard may be cut; up to ONE_LAUNCH_MAX_SPLITS the step of all ranks is one launch
+    from triton_distributed_b200.parallel.sp_flash_decode import ONE_LAUNCH_MAX_SPLITS, pick_shard_splits
+
+    lengths = (64, 512, 2048, 8192, 16384, 131072)
+    want = {(1, 8): (1, 8, 16, 32, 46, 55), (2, 8): (1, 8, 16, 27, 27, 27), (4, 8): (1, 8, 13, 13, 13, 13), (8, 8): (1, 6, 6, 6, 6, 6),
+            (16, 8): (1, 3, 3, 3, 3, 3), (64, 8): (1,) * 6, (1, 1): (1, 8, 16, 32, 46, 64)}
+    for (batch, heads), splits in want.items():
+        assert tuple(pick_shard_splits(batch, heads, 1, n) for n in lengths) == splits
+        if batch * heads >= 32:
+            assert all(s <= ONE_LAUNCH_MAX_SPLITS for s in splits)

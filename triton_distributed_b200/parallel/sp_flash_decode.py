@@ -16,12 +16,21 @@ from typing import Optional
 import torch
 
 from .. import _native
-from ..ops.attention import attention_reference, decode_workspace, merge_attention_partials, pick_kv_splits
+from ..ops.attention import attention_reference, decode_workspace, merge_attention_partials
 from ..ops.common import new_ctx_dev, ref_all_gather
 from ..runtime import get_runtime
 
 
 ONE_LAUNCH_MAX_SPLITS = 16
+
+
+def pick_shard_splits(batch: int, num_kv_heads: int, head_dim_chunks: int, positions: int, num_sms: int = 148) -> int:
+    """KV splits of this rank's shard: about sqrt(8 x blocks of 64 tokens), at most what fits one wave (three CTAs per SM) and 64.  A
+    rule of its own, not that of single-GPU decoding: the count also decides between one launch and two (see ``one_launch``), so a batch
+    that fills the GPU with few splits must not be cut further (8 x 8 heads x 8192 tokens: 6 splits and one launch)."""
+    blocks = max(1, (positions + 63) // 64)
+    one_wave = max(1, (3 * num_sms) // max(1, batch * num_kv_heads * head_dim_chunks))
+    return max(1, min(math.ceil(math.sqrt(8.0 * blocks)), one_wave, blocks, 64))
 
 
 class SpGQAFlashDecodeAttention:
@@ -43,8 +52,8 @@ class SpGQAFlashDecodeAttention:
         self.workspace = None
         self.counters = None
         # None: one launch while the local KV is cut into at most ONE_LAUNCH_MAX_SPLITS splits.  Beyond that the merge of
-        # the splits by a single CTA per KV head costs more than the second launch saves (bs 1, 16 k KV per rank, 45
-        # splits, two B200: 39 us in one launch, 34 us in two).  True / False force a form.
+        # the splits by a single CTA per KV head costs more than the second launch saves (bs 1, 16 k KV per rank, cut into
+        # 45, two B200: 39 us in one launch, 34 us in two).  True / False force a form.
         self.one_launch: Optional[bool] = None
         self.last_launches = 0
         if self.rt.is_cuda and num_ranks > 1:
@@ -74,7 +83,7 @@ class SpGQAFlashDecodeAttention:
         if B > self.max_batch:
             raise ValueError(f"batch {B} exceeds max_allowed_batch {self.max_batch}")
         group = Hq // self.num_kv_heads
-        splits = pick_kv_splits(B, self.num_kv_heads, (group + 15) // 16, k_cache.shape[1] * block_table.shape[1])
+        splits = pick_shard_splits(B, self.num_kv_heads, (group + 15) // 16, k_cache.shape[1] * block_table.shape[1])
         need = B * Hq * splits * (D + 1)
         if self.workspace is None or self.workspace.numel() < need:
             self.workspace = decode_workspace(B, Hq, D, splits, q.device)
