@@ -137,3 +137,17 @@ def test_flash_decode_shard_splits_and_launch_form():
         assert tuple(pick_shard_splits(batch, heads, 1, n) for n in lengths) == splits
         if batch * heads >= 32:
             assert all(s <= ONE_LAUNCH_MAX_SPLITS for s in splits)
+
+
+def test_decode_splits():
+    # one CTA per SM down to single blocks, one wave of short pieces, several waves of long ones or where one wave is not enough; none empty
+    from triton_distributed_b200.ops import pick_kv_splits
+
+    for args, want in {(1, 8, 1, 1024): 16, (1, 8, 1, 4096): 16, (4, 8, 1, 4096): 13, (8, 8, 1, 4096): 6, (16, 8, 1, 4096): 3, (16, 8, 1, 16384): 10,
+                       (64, 8, 1, 4096): 3, (32, 8, 1, 1024): 1, (1, 1, 1, 1): 1, (1, 8, 1, 32768): 32}.items():
+        assert pick_kv_splits(*args) == want, args
+    assert pick_kv_splits(48, 4, 1, 2048, head_dim=256) == 2 and pick_kv_splits(16, 4, 1, 2048, head_dim=64) == 8
+    for ctas in (1, 7, 32, 100, 500):
+        for n in (1, 63, 65, 1000, 4097, 100000):
+            blocks, splits = (n + 63) // 64, pick_kv_splits(ctas, 1, 1, n)
+            assert 1 <= splits <= min(blocks, 64) and (splits - 1) * -(-blocks // splits) < blocks

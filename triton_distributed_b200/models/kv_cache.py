@@ -25,7 +25,7 @@ class KV_Cache:
         self.block_table = torch.arange(batch_size, dtype=torch.int32, device=dev).unsqueeze(1).contiguous()
         self._row_base = (torch.arange(batch_size, dtype=torch.int64, device=dev) * max_length)
         self._ws = None
-        self.kv_splits = pick_kv_splits(batch_size, kv_heads, 1, max_length)
+        self.kv_splits = pick_kv_splits(batch_size, kv_heads, 1, max_length, head_dim=head_dim)
 
     # -- views used by the attention layer --------------------------------------------------------------------
     def layer(self, i: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -92,7 +92,7 @@ class PagedKVCache:
         self.block_table = order.to(torch.int32).reshape(batch_size, self.pages_per_seq).contiguous()
         self.kv_offset = torch.zeros(batch_size, dtype=torch.int32, device=dev)
         self._ws = None
-        self.kv_splits = pick_kv_splits(batch_size, kv_heads, 1, max_length)
+        self.kv_splits = pick_kv_splits(batch_size, kv_heads, 1, max_length, head_dim=head_dim)
 
     def layer(self, i: int):
         return self.k_cache[i], self.v_cache[i]

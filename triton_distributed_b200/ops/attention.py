@@ -172,19 +172,27 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                                return_lse, sink)
 
 
-def pick_kv_splits(batch: int, num_kv_heads: int, head_dim_chunks: int, max_kv_len: int, num_sms: int = 148) -> int:
+def pick_kv_splits(batch: int, num_kv_heads: int, head_dim_chunks: int, max_kv_len: int, num_sms: int = 148, head_dim: int = 128) -> int:
     """Number of KV splits: the larger of two wants.  While one CTA per SM is not reached, as many splits as that takes, down to a
     single 64-token block each (4 sequences x 4 heads x 512 tokens: 5.7 us with 8 splits, 7.2 with 2).  Beyond, splits of at least
-    four blocks up to three waves of the three CTAs an SM holds: the last wave and sequences of unequal length cost less when the
-    pieces are small, the merge more (64 x 8 heads x 4096 tokens: 148 us with 1 split, 132 with 3, 139 with 6; 8 x 4 x 2048: 20.0 us
-    with 3, 13.9 with 8, 17.5 with 16).  Above 32 the merge is a launch of its own (1 x 8 x 32768: 30.6 us with 32 splits, 38 with
-    55), worth it only where 32 splits leave SMs idle.  At most 64."""
+    four blocks up to nine CTAs per SM: the last wave and sequences of unequal length cost less when the pieces are small, the merge
+    more (64 x 8 heads x 4096 tokens, lengths from half of that: 167 us with 1 split, 139 with 3).  But no second, partly filled wave
+    of short pieces where one wave (three CTAs per SM with heads of 128, one with heads of 256) takes the problem: 4 x 8 x 4096: 21.6
+    us with 13 splits, 27.5 with 16; heads of 256, 24 x 8 x 2048: 95 with 2, 126 with 7.  Pieces of ten blocks and more hide it
+    (16 x 8 x 16384, unequal: 152 with 3, 141 with 10), with heads of 256 of sixteen (20 x 4 x 6000: 132 with 1, 82 with 5, 104 with 17).  Above 32 the merge is a launch of its own (1 x 8 x 32768: 30.6 us with 32
+    splits, 38 with 55), worth it only where 32 splits leave SMs idle.  At most 64."""
     blocks = max(1, (max_kv_len + 63) // 64)
     ctas = max(1, batch * num_kv_heads * head_dim_chunks)
     one_each = min(blocks, num_sms // ctas)
     waves = min(blocks // 4, (9 * num_sms + ctas // 2) // ctas)
     cap = FUSED_COMBINE_MAX_SPLITS if ctas * FUSED_COMBINE_MAX_SPLITS >= num_sms else 64
-    return max(1, min(max(one_each, waves), cap))
+    splits = max(1, min(max(one_each, waves), cap))
+    wave = max(1, min(5, 384 // head_dim)) * num_sms
+    if splits * ctas > wave and head_dim > 128:
+        splits = min(splits, max(wave // ctas, one_each, blocks // 16, 1))
+    elif splits * ctas > wave and blocks < 10 * splits and ctas <= 3 * num_sms:
+        splits = min(splits, max(wave // ctas, one_each, 1))
+    return -(-blocks // -(-blocks // splits))      # none without a block
 
 
 FUSED_COMBINE_MAX_SPLITS = 32   # up to here the last split CTA merges the partials itself; beyond, a combine launch
@@ -222,7 +230,7 @@ def gqa_fwd_batch_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
         Hkv = k_cache.shape[2]
         group = Hq // Hkv
         splits = kv_split if kv_split > 0 else pick_kv_splits(B, Hkv, (group + 15) // 16,
-                                                                k_cache.shape[1] * block_table.shape[1])
+                                                                k_cache.shape[1] * block_table.shape[1], head_dim=D)
         need = B * Hq * splits * (D + 1)
         if workspace is None or workspace.numel() < need:
             workspace = decode_workspace(B, Hq, D, splits, q.device)
