@@ -335,6 +335,14 @@ def test_delta_rule_many_heads(rt, shape):
     r.check()
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 96, 64, 4), (9, 3, 96, 128, 4), (20, 4, 96, 72, 2), (3, 1, 128, 80, 3), (40, 4, 128, 128, 4), (9, 9, 80, 128, 4)])
+def test_delta_rule_state_forms(rt, shape):
+    # one wave of 16, 32 or 64 columns and more than a wave, with the matrices of a chunk in registers or in shared memory
+    r = Rule(*shape, lens=[70, 130, 1, 64])
+    r.run([(s, 0, n) for s, n in enumerate(r.lens)], "chunk")
+    r.check()
+
+
 @pytest.mark.parametrize("shape", RULES)
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_delta_rule_portions_and_decoding(rt, shape, dtype):

@@ -382,19 +382,24 @@ __global__ void __launch_bounds__(kThreads, 2) delta_local_kernel(const DeltaArg
 // ---------------------------------------------------------------------------------------------------- sequential part
 // KS: 16-row blocks of dk, a warp each; NT: tiles of eight columns per CTA.  Every CTA of a head reads the whole of trans, which is
 // most of the traffic and what the pass is bound by: with 32 columns a CTA 96 heads of 128 x 128 over 6001 tokens moved 983 MB
-// from L2 in 259 us, with 64 columns 590 MB in 187.  A lane reads exactly the fragments it has copied, so trans waits in a ring of
-// two chunks of shared memory without a barrier (as registers it left no room for 64 columns).
+// from L2 in 259 us, with 64 columns 590 MB in 187.  trans arrives ahead, in registers (one chunk) or, without a barrier, since a
+// lane reads exactly the fragments it has copied, in a ring of two chunks of shared memory.  Heads of 128 have no registers left
+// for it (the whole call over 4096 tokens with 8 heads: 248 us with registers, 218 with the ring; 32 heads, 32 columns a CTA: 598 and
+// 545).  Smaller heads have, and pay for the trip through shared memory (8192 tokens, 12 heads of 64: 347 and 441); heads of 96 lie
+// between (14 heads of one wave: 166 and 154, 30 heads with 32 columns a CTA: 254 and 273).
 constexpr int kTransRing = 2;
 template <int KS, int NT>
+constexpr bool state_ring() { return KS == 8 || (KS == 6 && NT != 4); }
+template <int KS, int NT>
 constexpr size_t state_smem() {
-  return static_cast<size_t>(2 * 2 * KS * 16 * (NT * 8 + 8) * 2) + (KS <= 8 ? static_cast<size_t>(kTransRing) * KS * KS * 64 * 16 : 0);
+  return static_cast<size_t>(2 * 2 * KS * 16 * (NT * 8 + 8) * 2) + (state_ring<KS, NT>() ? static_cast<size_t>(kTransRing) * KS * KS * 64 * 16 : 0);
 }
 
 template <int KS, int NT>
 __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs p) {
   extern __shared__ __align__(16) uint8_t smem[];
   constexpr int kPitch = NT * 8 + 8;
-  constexpr bool kRing = KS <= 8;           // larger heads read trans where it lies
+  constexpr bool kRing = state_ring<KS, NT>(), kAhead = KS <= 8 && !kRing;        // larger heads read trans where it lies
   constexpr int ksteps = KS;
   constexpr int part = KS * 16 * kPitch;
   const int vtiles = p.dv >> 3;
@@ -421,24 +426,34 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
   const float4* inject = reinterpret_cast<const float4*>(p.inject) + (static_cast<int64_t>(warp) * vtiles + tile0) * 32 + lane;
   uint4* states = reinterpret_cast<uint4*>(p.states) + (static_cast<int64_t>(warp) * vtiles + tile0) * 32 + lane;
   const int64_t tr_step = static_cast<int64_t>(ksteps) * ksteps * 64, in_step = static_cast<int64_t>(ksteps) * vtiles * 32;
+  uint4 nh[kAhead ? KS : 1], nl[kAhead ? KS : 1];
   float4 ni[NT] = {};
   float nd = 0.f;
-  auto fetch = [&](int c) {                 // inject to registers, a chunk ahead
+  auto fetch = [&](int c) {                 // inject, and without the ring trans, to registers, a chunk ahead
     if (c >= c1) return;
     const int64_t ch = static_cast<int64_t>(c) * p.H + h;
     nd = p.decay[ch];
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        nh[ks] = trans[ch * tr_step + ks * 64];
+        nl[ks] = trans[ch * tr_step + ks * 64 + 32];
+      }
+    }
 #pragma unroll
     for (int j = 0; j < NT; ++j)
       if (j < tiles) ni[j] = inject[ch * in_step + j * 32];
   };
   auto copy = [&](int c) {                  // trans to the ring, one group per chunk
-    if (kRing && c < c1) {
-      const uint4* src = trans + (static_cast<int64_t>(c) * p.H + h) * tr_step;
-      uint4* dst = ring + (c - c0) % kTransRing * tr_step;
+    if constexpr (kRing) {
+      if (c < c1) {
+        const uint4* src = trans + (static_cast<int64_t>(c) * p.H + h) * tr_step;
+        uint4* dst = ring + (c - c0) % kTransRing * tr_step;
 #pragma unroll
-      for (int i = 0; i < 2 * KS; ++i) attn::cp_async16(dst + i * 32, src + i * 32, true);
+        for (int i = 0; i < 2 * KS; ++i) attn::cp_async16(dst + i * 32, src + i * 32, true);
+      }
+      cp_async_commit();
     }
-    cp_async_commit();
   };
   copy(c0);
   copy(c0 + 1);
@@ -464,13 +479,28 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
       lo1[j][0] = lo1[j][1] = lo1[j][2] = lo1[j][3] = 0.f;
       lo2[j][0] = lo2[j][1] = lo2[j][2] = lo2[j][3] = 0.f;
     }
+    uint4 th[kAhead ? KS : 1], tl[kAhead ? KS : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        th[ks] = nh[ks];
+        tl[ks] = nl[ks];
+      }
+    }
     fetch(c + 1);
-    cp_async_wait<kTransRing - 1>();
+    if constexpr (kRing) cp_async_wait<kTransRing - 1>();
     __syncthreads();       // the other buffer is free as well: its readers have passed this barrier
     const uint4* A = kRing ? ring + (c - c0) % kTransRing * tr_step : trans + ch * tr_step;
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
-      const uint4 fh = A[ks * 64], fl = A[ks * 64 + 32];
+      uint4 fh, fl;
+      if constexpr (kAhead) {
+        fh = th[ks];
+        fl = tl[ks];
+      } else {
+        fh = A[ks * 64];
+        fl = A[ks * 64 + 32];
+      }
       const uint32_t ah[4] = {fh.x, fh.y, fh.z, fh.w}, al[4] = {fl.x, fl.y, fl.z, fl.w};
       const int brow = (ks * 16 + (mat & 1) * 8 + mr) * kPitch + (mat >> 1) * 8;
 #pragma unroll
@@ -496,7 +526,7 @@ __global__ void __launch_bounds__(32 * KS, 1) delta_state_kernel(const DeltaArgs
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[j][e] = acc[j][e] + (lo1[j][e] + lo2[j][e]);
   }
-  cp_async_wait<0>();
+  if constexpr (kRing) cp_async_wait<0>();
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
     if (j >= tiles) break;
@@ -633,21 +663,23 @@ cudaError_t launch_state(const DeltaArgs& a, cudaStream_t s) {
 }
 template <int NT>
 cudaError_t launch_state_nt(const DeltaArgs& a, cudaStream_t s) {
+  if constexpr (NT <= 4) {
+    switch (a.dk / 16) {
+      case 1: return launch_state<1, NT>(a, s);
+      case 2: return launch_state<2, NT>(a, s);
+      case 3: return launch_state<3, NT>(a, s);
+      case 4: return launch_state<4, NT>(a, s);
+      case 5: return launch_state<5, NT>(a, s);
+      case 12: return launch_state<12, NT>(a, s);
+      case 16: return launch_state<16, NT>(a, s);
+      default: break;
+    }
+  }
   switch (a.dk / 16) {
-    case 1: return launch_state<1, NT>(a, s);
-    case 2: return launch_state<2, NT>(a, s);
-    case 3: return launch_state<3, NT>(a, s);
-    case 4: return launch_state<4, NT>(a, s);
-    case 5: return launch_state<5, NT>(a, s);
     case 6: return launch_state<6, NT>(a, s);
     case 8: return launch_state<8, NT>(a, s);
-    default: break;
+    default: return cudaErrorInvalidValue;
   }
-  if constexpr (NT <= 4) {
-    if (a.dk == 192) return launch_state<12, NT>(a, s);
-    if (a.dk == 256) return launch_state<16, NT>(a, s);
-  }
-  return cudaErrorInvalidValue;
 }
 template <int TW>
 cudaError_t launch_out(const DeltaArgs& a, cudaStream_t s) {
@@ -675,14 +707,18 @@ cudaError_t launch_delta_chunk(const DeltaArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   e = launch_pdl(delta_local_kernel, dim3(a.NC, a.H), dim3(kThreads), local_smem(a.dk), s, a);
   if (e != cudaSuccess) return e;
-  // every CTA of a head reads the same operands: narrower column tiles only while they still fit one wave
+  // Every CTA of a head reads the same operands: column tiles as narrow as one wave allows.  Beyond a wave of 64 columns 32 again, for
+  // the last wave and unequal sequences (32 heads of 128, 6001 tokens: three sequences 841 us with 64 columns, 787 with 32, two, a wave of
+  // 64 columns, 781 and 780; 40 heads, one sequence: 749 and 761).  Heads of 96, whose form of 32 columns has trans in registers, stay at
+  // 64 (266 and 269 us); smaller heads have no such form (24 heads of 64, three sequences: 414 us with 64 columns, 394 with 32).
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t heads = static_cast<int64_t>(a.N) * a.H;
-  e = heads * ((a.dv + 15) / 16) <= sms                   ? launch_state_nt<2>(a, s)
-      : heads * ((a.dv + 31) / 32) <= sms || a.dk > 128 ? launch_state_nt<4>(a, s)
-                                                          : launch_state_nt<8>(a, s);
+  auto one_wave = [&](int cols) { return heads * ((a.dv + cols - 1) / cols) <= sms; };
+  e = one_wave(16)                                                     ? launch_state_nt<2>(a, s)
+      : !one_wave(32) && (a.dk == 96 || (a.dk == 128 && one_wave(64))) ? launch_state_nt<8>(a, s)
+                                                                       : launch_state_nt<4>(a, s);
   if (e != cudaSuccess) return e;
   if (a.dv <= 64) return launch_out<4>(a, s);
   if (a.dv <= 128) return launch_out<8>(a, s);
