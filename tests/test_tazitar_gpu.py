@@ -1,5 +1,6 @@
 """Tazitar on one GPU: every kernel alone and the whole model (bf16 and fp32) against the plain oracle on the CPU."""
 import json
+import math
 import os
 import subprocess
 import sys
@@ -341,6 +342,24 @@ def test_delta_rule_state_forms(rt, shape):
     r = Rule(*shape, lens=[70, 130, 1, 64])
     r.run([(s, 0, n) for s, n in enumerate(r.lens)], "chunk")
     r.check()
+
+
+@pytest.mark.parametrize("impl", ["chunk", "recurrent"])
+def test_delta_rule_gates_far_below_zero(rt, impl):
+    # the read-out times silu(gate): what is left of it down to the smallest numbers, against a gate of two
+    r = Rule(3, 3, 64, 64, 2, lens=[66])
+    outs = {}
+    for gate in (2.0, -20.0, -60.0, -80.0, -88.0):
+        r.z[:, -3 * 64:] = gate
+        r.run([(0, 0, 66)], impl)
+        outs[gate] = r.out.double().clone()
+    silu = lambda x: x / (1 + math.exp(-x))   # noqa: E731
+    for gate in (-20.0, -60.0, -80.0, -88.0):
+        # one rounding to bf16 on each side, of what bf16 holds with all its bits
+        want = outs[2.0] / silu(2.0)
+        seen = want.abs() > 0.1
+        assert seen.float().mean() > 0.5
+        torch.testing.assert_close(outs[gate][seen] / silu(gate), want[seen], rtol=2 ** -7, atol=0)
 
 
 @pytest.mark.parametrize("shape", RULES)
