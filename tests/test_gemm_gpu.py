@@ -254,6 +254,34 @@ def test_gemm_chunks_without_a_store(M, N, form):
         torch.testing.assert_close(out.double(), ref, rtol=2 ** -8, atol=2 ** -10)
 
 
+@pytest.mark.parametrize("form", ["pair", "gemv", "grouped"])
+def test_swiglu_gate_range(form):
+    # SiLU in the epilogues for gates from -100 to 40, down to the smallest results
+    from triton_distributed_b200 import ops
+
+    z = torch.cat([torch.linspace(-100, -80, 121), torch.linspace(-80, 40, 391)]).to("cuda", torch.bfloat16)
+    M, F, K = (16, 32, 8) if form == "gemv" else (512, 256, 8) if form == "pair" else (512, 64, 8)
+    out = []
+    for rows in z.split(M):
+        x = torch.zeros(rows.numel(), K, device="cuda", dtype=torch.bfloat16)
+        x[:, 0], x[:, 1] = rows, 1
+        w = torch.zeros(2 * F, K, device="cuda", dtype=torch.bfloat16)
+        w[:F, 0], w[F:, 1] = 1, 1.5
+        if form == "gemv":
+            y = ops.gemv_fused(x, w, swiglu=True)
+        elif form == "pair":
+            y = ops.gemm_swiglu(x, w)
+        else:
+            srt = ops.sort_topk_ids_align_block_size(torch.zeros(rows.numel(), 1, device="cuda", dtype=torch.int32), 1)
+            y = ops.group_gemm_gather(x, w.unsqueeze(0), srt, a_row_div=1, scatter_out=True, gated=True)
+        out.append(y)
+    torch.cuda.synchronize()
+    y = torch.cat(out).double()
+    ref = (torch.nn.functional.silu(z.double()) * 1.5).unsqueeze(1).expand_as(y)
+    # one rounding to bf16; below the smallest normal number of bf16 results may be flushed
+    torch.testing.assert_close(y, ref, rtol=2 ** -8, atol=1.2e-38)
+
+
 @pytest.mark.parametrize("M,F,K", [(1, 4, 8), (1, 3, 264), (2, 1001, 520), (4, 12288, 256), (7, 149, 2048), (16, 300, 4096), (1, 70, 40000)])
 def test_gemv_swiglu(M, F, K):
     # groups of four gate and four up rows: whole, shared by warps, partly empty
