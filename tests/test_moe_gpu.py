@@ -199,6 +199,26 @@ def test_group_gemm_partial_column_tiles(rt, N, gated):
             torch.testing.assert_close(y[at], ref, rtol=2 ** -8, atol=2 ** -10)
 
 
+@pytest.mark.parametrize("T,E,k,H,I", [(5, 4, 2, 64, 16), (300, 6, 3, 320, 136)])
+def test_sorted_rows_that_end_behind_the_last_in_use(rt, T, E, k, H, I):
+    # the sorted layout has room for the worst case; x may hold the padded rows in use only
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(T)
+    w2 = (torch.randn(E, H, I, device="cuda") * I ** -0.5).to(torch.bfloat16)
+    ids = torch.rand(T, E, device="cuda").topk(k).indices.to(torch.int32)
+    rw = torch.rand(T, k, device="cuda")
+    srt = ops.sort_topk_ids_align_block_size(ids, E)
+    used = int(srt.meta[0])
+    assert used < srt.sorted_ids.numel()
+    x = torch.randn(srt.sorted_ids.numel(), I, device="cuda", dtype=torch.bfloat16)
+    ctx = ops.create_moe_ar_context(max_token_num=T, hidden_dim=H, num_experts=E, topk=k)
+    whole, part = (ops.group_gemm_gather(t, w2, srt, a_row_div=0, row_weight=rw)[srt.pos_of.long()] for t in (x, x[:used].clone()))
+    whole_r, part_r = (ops.run_moe_reduce_ar(t, w2, ids, rw, ctx, sort=srt) for t in (x, x[:used].clone()))
+    torch.cuda.synchronize()
+    assert torch.equal(whole, part) and torch.equal(whole_r, part_r)
+
+
 @pytest.mark.parametrize("E", [1, 31, 128, 129, 512])
 def test_router_bf16_logits(E):
     from triton_distributed_b200.ops import topk_router

@@ -183,7 +183,6 @@ void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor
   TORCH_CHECK(y.is_cuda() && y.scalar_type() == at::kBFloat16 && y.dim() == 2 && y.stride(1) == 1, "moe_fused: bf16 y");
   const int64_t K = x.size(1), E = w.size(0), N = w.size(1);
   TORCH_CHECK(w.size(2) == K && y.size(1) == (gated ? N / 2 : N) && (!gated || N % 2 == 0), "moe_fused: shape mismatch");
-  TORCH_CHECK(a_row_div > 0 || x.size(0) >= sorted_ids.numel(), "moe_fused: x must hold every sorted row");
   TORCH_CHECK(sorted_ids.scalar_type() == at::kInt && tile_expert.scalar_type() == at::kInt && meta.scalar_type() == at::kInt,
               "moe_fused: int32 index tensors expected");
   TORCH_CHECK(sorted_ids.numel() == tile_expert.numel() * 128, "moe_fused: sorted_ids must hold 128 rows per tile");
@@ -191,6 +190,7 @@ void fill_moe_common(tdb::MoeFusedArgs& g, const at::Tensor& x, const at::Tensor
   g.K = K; g.N = N; g.k_top = k_top;
   g.x = x.data_ptr();
   g.ldx = x.stride(0);
+  g.x_rows = x.size(0);
   g.a_row_div = a_row_div;
   g.gated = gated ? 1 : 0;
   g.sorted_ids = sorted_ids.data_ptr<int32_t>();

@@ -54,6 +54,7 @@ struct MoeFusedArgs {
   int K, N, k_top;
   const void* x;               // bf16 source rows [rows, ldx]; all-gather mode: the local token shard [t_local, ldx = K]
   int64_t ldx;
+  int64_t x_rows;              // rows of x (read for a_row_div = 0, whose x may end behind the last row in use)
   int a_row_div;               // source row of sorted row r = sorted_ids[r] / a_row_div; 0: row r itself (not all-gather)
   int gated;                   // plain mode: w = gate rows then up rows, y [*, N / 2] = silu(gate) * up
   const int32_t* sorted_ids;   // [max_tiles * 128]

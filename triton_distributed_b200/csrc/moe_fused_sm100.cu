@@ -72,6 +72,7 @@ struct MoeParams {
   const __nv_bfloat16* x;      // A source rows: [tokens or pairs, K]; all-gather mode: the local shard [t_local, K]
   int64_t ldx;
   int a_row_div;               // source row of sorted row r: sorted_ids[r] / a_row_div (k for token rows, 1 for pair rows), 0: row r
+  int64_t x_rows;              // rows of x; a_row_div = 0: sorted rows beyond them read as zeros
   int gated;                   // weights are gate rows, then up rows: a tile holds 128 of each, y = silu(gate) * up has N / 2 columns
   const int32_t* sorted_ids;   // [cap] flat pair index per sorted row, -1 = padding
   const int32_t* tile_expert;  // [cap / 128]
@@ -648,6 +649,7 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
           src[i] = nullptr;
           if (id >= 0) {
             const int64_t srow = p.a_row_div > 0 ? id / p.a_row_div : mt * kBM + r;
+            if (p.a_row_div == 0 && srow >= p.x_rows) continue;
             if (p.mode == kMoeAllGather) {
               const int owner = static_cast<int>(srow / p.t_local);
               const int lrow = static_cast<int>(srow - static_cast<int64_t>(owner) * p.t_local);
@@ -734,6 +736,7 @@ cudaError_t launch_moe_fused(const MoeFusedArgs& a, cudaStream_t stream) {
   p.K = a.K; p.N = a.N; p.k_top = a.k_top;
   p.x = reinterpret_cast<const __nv_bfloat16*>(a.x);
   p.ldx = a.ldx;
+  p.x_rows = a.x_rows;
   p.a_row_div = a.a_row_div;
   p.sorted_ids = a.sorted_ids;
   p.tile_expert = a.tile_expert;

@@ -325,7 +325,7 @@ def group_gemm_gather(x: torch.Tensor, w: torch.Tensor, srt: MoESort, a_row_div:
                       out: Optional[torch.Tensor] = None, gated: bool = False) -> torch.Tensor:
     """Grouped GEMM whose A rows are gathered inside the kernel: sorted row r multiplies ``x[sorted_ids[r] // a_row_div]``
     (``a_row_div = k`` when ``x`` holds tokens, 1 when it holds (token, slot) pairs, 0 when its row r already is sorted
-    row r) with its tile's expert weight.  ``gated``: ``w`` holds gate rows, then up rows, and the result is
+    row r; it may end behind the last row in use) with its tile's expert weight.  ``gated``: ``w`` holds gate rows, then up rows, and the result is
     ``silu(gate) * up`` [*, N / 2].
     Output in the sorted layout [cap, N], or in (token, slot) order [pairs, N] when ``scatter_out``; ``row_weight``
     [pairs] scales every row in the epilogue."""
