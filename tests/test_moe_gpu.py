@@ -219,6 +219,23 @@ def test_sorted_rows_that_end_behind_the_last_in_use(rt, T, E, k, H, I):
     assert torch.equal(whole, part) and torch.equal(whole_r, part_r)
 
 
+def test_padding_rows_are_zeros_whatever_lies_in_x(rt):
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(1)
+    T, E, k, I = 200, 5, 2, 96
+    ids = torch.rand(T, E, device="cuda").topk(k).indices.to(torch.int32)
+    srt = ops.sort_topk_ids_align_block_size(ids, E)
+    pad, used = srt.sorted_ids < 0, int(srt.meta[0])
+    x = torch.randn(pad.numel(), I, device="cuda", dtype=torch.bfloat16)
+    x[pad] = float("nan")
+    for N, gated in ((320, False), (400, True)):
+        w = (torch.randn(E, N, I, device="cuda") * I ** -0.5).to(torch.bfloat16)
+        y = ops.group_gemm_gather(x, w, srt, a_row_div=0, gated=gated)
+        torch.cuda.synchronize()
+        assert (y[:used][pad[:used]] == 0).all() and torch.isfinite(y[srt.pos_of.long()]).all()
+
+
 @pytest.mark.parametrize("E", [1, 31, 128, 129, 512])
 def test_router_bf16_logits(E):
     from triton_distributed_b200.ops import topk_router

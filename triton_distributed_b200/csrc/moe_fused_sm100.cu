@@ -558,7 +558,8 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         if (p.scatter_out) {
           if (id >= 0) dst = p.y + static_cast<int64_t>(id) * p.ldy;
         } else {
-          dst = p.y + static_cast<int64_t>(srow) * p.ldy;   // padding rows are written too (zeros): the layout stays dense
+          // padding rows are written too, as zeros: the layout stays dense.  By TMA they are read too, whatever lies there.
+          dst = p.y + static_cast<int64_t>(srow) * p.ldy;
         }
         // 64 columns of the row at a time, as eight 16-byte pieces
         const int chunks = (p.gated ? kBN / 2 : kBN) / kEpiCols, width = p.gated ? p.N >> 1 : p.N;
@@ -597,6 +598,7 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
               o.y = pack_bf16x2(wgt * __uint_as_float(r[8 * j + 2]), wgt * __uint_as_float(r[8 * j + 3]));
               o.z = pack_bf16x2(wgt * __uint_as_float(r[8 * j + 4]), wgt * __uint_as_float(r[8 * j + 5]));
               o.w = pack_bf16x2(wgt * __uint_as_float(r[8 * j + 6]), wgt * __uint_as_float(r[8 * j + 7]));
+              if (id < 0) o = make_uint4(0u, 0u, 0u, 0u);
               const int piece = 4 * h + j;
               if (p.tma_y) *reinterpret_cast<uint4*>(stg + row_in_tile * 128 + ((piece ^ (row_in_tile & 7)) << 4)) = o;
               else if (dst != nullptr && col0 + 8 * piece + 8 <= width) st_v4(dst + col0 + 8 * piece, o);
