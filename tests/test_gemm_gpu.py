@@ -254,6 +254,21 @@ def test_gemm_chunks_without_a_store(M, N, form):
         torch.testing.assert_close(out.double(), ref, rtol=2 ** -8, atol=2 ** -10)
 
 
+@pytest.mark.parametrize("M,F,K", [(9, 256, 128), (128, 264, 200), (129, 256, 64), (200, 520, 72), (255, 256, 512), (256, 128, 64), (300, 252, 64)])
+def test_gemm_swiglu_two_launches(M, F, K):
+    # rows and widths on this side of the pair kernel's: every GEMM below it, then the activation
+    from triton_distributed_b200 import ops
+
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    g, u = (x.double() @ w.double().t()).chunk(2, dim=-1)
+    out = ops.gemm_swiglu(x, w)
+    torch.cuda.synchronize()
+    # gate, up and result are rounded to bf16
+    torch.testing.assert_close(out.double(), torch.nn.functional.silu(g) * u, rtol=2 ** -6, atol=2 ** -8)
+
+
 @pytest.mark.parametrize("form", ["pair", "gemv", "grouped"])
 def test_swiglu_gate_range(form):
     # SiLU in the epilogues for gates from -100 to 40, down to the smallest results

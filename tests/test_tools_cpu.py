@@ -233,3 +233,18 @@ def test_op_log_records_json(tmp_path):
     assert new and new[-1]["op"] == "gemm" and new[-1]["shape"] == {"M": 8, "N": 16, "K": 64}
     rec = json.loads(path.read_text().splitlines()[-1])
     assert rec["us"] > 0 and "tflops" in rec and "roofline_frac" in rec
+
+
+def test_op_log_counts_a_product_once():
+    # gemm_swiglu is one record: its own where it is one launch, else its GEMM's
+    import torch
+    from triton_distributed_b200 import ops
+    from triton_distributed_b200.utils import oplog
+
+    oplog.enable()
+    try:
+        ops.gemm_swiglu(torch.randn(3, 8), torch.randn(16, 8))
+        ops.gemm_swiglu(torch.randn(300, 8), torch.randn(16, 8))
+        assert [r["op"] for r in oplog.flush()] == ["gemm", "gemm"]
+    finally:
+        oplog.disable()

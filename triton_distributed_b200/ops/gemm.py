@@ -110,14 +110,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, b
     return res
 
 
-@logged_op("gemm_swiglu", _gemm_meta)
+GEMM_SWIGLU_MIN_ROWS = 256      # rows that fill a tile of the pair kernel
+
+
 def gemm_swiglu(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``a`` [M, K], ``w`` [2 F, K] (gate rows, then up rows) -> ``silu(a gate^T) * (a up^T)`` [M, F].  From 256 rows on
     one launch of the CTA-pair kernel with the activation in its epilogue; fewer rows are a GEMM and an activation."""
-    M, N = a.numel() // a.shape[-1], w.shape[0]
-    if not (M >= 256 and N >= 512 and N % 16 == 0 and _native.use_native(a, w) and a.dtype == torch.bfloat16
+    if a.numel() < GEMM_SWIGLU_MIN_ROWS * max(a.shape[-1], 1):
+        return silu_mul(gemm(a, w))
+    N = w.shape[0]
+    if not (N >= 512 and N % 16 == 0 and _native.use_native(a, w) and a.dtype == torch.bfloat16
             and a.stride(-1) == 1 and w.stride(-1) == 1 and os.environ.get("TDB200_GEMM_PAIR", "1") != "0"):
         return silu_mul(gemm(a, w))
+    return _gemm_swiglu_pair(a, w)
+
+
+@logged_op("gemm_swiglu", _gemm_meta)
+def _gemm_swiglu_pair(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    M, N = a.numel() // a.shape[-1], w.shape[0]
     out = torch.empty((*a.shape[:-1], N // 2), dtype=a.dtype, device=a.device)
     _native.load(True).gemm_bf16(a.reshape(M, a.shape[-1]), w, out.view(M, N // 2), 512, 0, None, True)
     return out

@@ -101,7 +101,11 @@ class TP_MLP:
 
     def dist_triton_gemm_ar_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """GEMM -> act -> fused GEMM+AllReduce (decode sizes); x replicated."""
-        h = ops.gemm_swiglu(x, self.gate_up_proj)
+        # gemm_swiglu's rule, asked here: a decode step is bound by its calls, and one more is a microsecond of 41
+        if x.numel() < 256 * self.hidden:
+            h = ops.silu_mul(ops.gemm(x, self.gate_up_proj))
+        else:
+            h = ops.gemm_swiglu(x, self.gate_up_proj)
         return ops.gemm_allreduce_op(self.gemm_ar_ctx, h, self.down_proj)
 
     # per-op entry points used by the layer benchmarks of the reference (tp_mlp.py:231-274)
