@@ -64,7 +64,17 @@ def test_gdn_chunk_kernels_over_column_tiles_and_sequence_ends(H, V, lens):
     o_r, s_r = ops.gated_delta_rule_recurrent(q, k, v, g, beta, K ** -0.5, h0, cu)
     cum = torch.cat([g[0, t:min(t + 64, b)].double().cumsum(0) for a, b in zip(cu.tolist(), cu.tolist()[1:]) for t in range(a, b, 64)])
     torch.testing.assert_close(gc[0].double(), cum, rtol=1e-5, atol=1e-5)
-    assert (A.triu(1) if T == 1 else A)[0, 0, 0, 1:].abs().max().item() == 0.0
+    # A of every chunk: the inverse of I + L, L = beta (k k^T) e^(gc_i - gc_j) below the diagonal, from what the kernel reads; its own
+    # sums are fp32 and so are those of the inverse, 64 terms of order one at most
+    for a, b in zip(cu.tolist(), cu.tolist()[1:]):
+        for t in range(a, b, 64):
+            n = min(t + 64, b) - t
+            kk, gg, bb = k[0, t:t + n].double().transpose(0, 1), gc[0, t:t + n].double().t(), beta[0, t:t + n].double().t()
+            L = ((kk @ kk.transpose(1, 2)) * bb[:, :, None] * torch.exp(gg[:, :, None] - gg[:, None, :])).tril(-1)
+            want = torch.linalg.inv(torch.eye(n, device="cuda", dtype=torch.float64) + L)
+            got = A[0, t:t + n].double().transpose(0, 1)
+            torch.testing.assert_close(got[:, :, :n], want, rtol=1e-4, atol=1e-5)
+            assert (got.triu(1) == 0).all()
     assert (o.float() - o_r).norm().item() < 2 ** -7 * o_r.norm().item()
     assert (ht - s_r).norm().item() < 2 ** -7 * s_r.norm().item()
     empty = [i for i, n in enumerate(lens) if n == 0]
