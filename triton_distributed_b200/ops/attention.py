@@ -9,6 +9,7 @@ cache ``[B, max_len, Hkv, D]`` is the case ``page_size = max_len`` with ``block_
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -172,6 +173,7 @@ def flash_attn_varlen(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                                return_lse, sink)
 
 
+@functools.lru_cache(maxsize=1024)      # numbers of numbers: 1.5 us of a decode call that is 12 in all
 def pick_kv_splits(batch: int, num_kv_heads: int, head_dim_chunks: int, max_kv_len: int, num_sms: int = 148, head_dim: int = 128) -> int:
     """Number of KV splits: the larger of two wants.  While one CTA per SM is not reached, as many splits as that takes, down to a
     single 64-token block each (4 sequences x 4 heads x 512 tokens: 5.7 us with 8 splits, 7.2 with 2).  Beyond, splits of at least

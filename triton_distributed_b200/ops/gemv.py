@@ -125,6 +125,8 @@ def gemv_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = N
                          ar_ctx.flags, ar_ctx.ctx_dev, ar_ctx.m_cap, ar_ctx.max_ctas, 0,
                          bool(ar_ctx.use_multimem and rt.has_multicast), rt.config.wait_timeout_s)
         ar_ctx.calls += 1
+    elif swiglu:
+        lib.gemv_bf16(x, w, out, norm_weight, float(eps), gated, residual, 0, True)
     else:
-        lib.gemv_bf16(x, w, out, norm_weight, float(eps), gated, residual, 0, bool(swiglu))
+        lib.gemv_bf16(x, w, out, norm_weight, float(eps), gated, residual, 0)
     return out
