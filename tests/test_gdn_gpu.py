@@ -96,3 +96,23 @@ def test_gdn_state_at_an_odd_address():
         want = ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, h0.clone(), True, cu, impl="chunk")
         torch.cuda.synchronize()
         assert torch.equal(got[1], want[1]) and torch.equal(got[3], want[3])
+
+
+def test_gdn_chunk_scratch():
+    """The intermediates of a call take no more than w, u, v_new and the chunk states in the form with row-major operands did."""
+    from test_gdn_cpu import _inputs
+    from triton_distributed_b200 import ops
+
+    T, H, K, V = 4096, 8, 128, 128
+    q, k, v, g, beta = _inputs(T, H, K, V, seed=2, dtype=torch.bfloat16, device="cuda")
+    cu = torch.tensor([0, T], dtype=torch.int32, device="cuda")
+    ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, None, False, cu, impl="chunk")
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = ops.chunk_gated_delta_rule_fwd(q, k, v, g, beta, K ** -0.5, None, False, cu, impl="chunk")
+    torch.cuda.synchronize()
+    chunks = (T // 64 + 1) * H
+    scratch = chunks * 2 * (64 * K + 2 * 64 * V + K * V)
+    # results, and the allocator's 512-byte and 2 MB roundings
+    assert torch.cuda.max_memory_allocated() - before <= scratch + T * H * (2 * V + 4) + (12 << 20), out[1].shape

@@ -305,7 +305,6 @@ std::vector<at::Tensor> gdn_chunk_fwd(const at::Tensor& q, const at::Tensor& k, 
   at::Tensor w = at::empty({NC, H, 64, K}, q.options());
   at::Tensor kd = at::empty({NC, H, K, 64}, q.options());
   at::Tensor u = at::empty({NC, H, 64, V}, q.options());
-  at::Tensor vn = at::empty({NC, H, 64, V}, q.options());
   at::Tensor hs = at::empty({NC, H, K, V}, q.options());
   tdb::GdnChunkArgs a;
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr();
@@ -316,7 +315,7 @@ std::vector<at::Tensor> gdn_chunk_fwd(const at::Tensor& q, const at::Tensor& k, 
   a.decay = decay.data_ptr<float>();
   a.g_cumsum = gc.data_ptr<float>();
   a.a_out = return_a ? A.data_ptr<float>() : nullptr;
-  a.w = w.data_ptr(); a.kd = kd.data_ptr(); a.u = u.data_ptr(); a.v_new = vn.data_ptr(); a.h_chunks = hs.data_ptr();
+  a.w = w.data_ptr(); a.kd = kd.data_ptr(); a.u = u.data_ptr(); a.v_new = u.data_ptr(); a.h_chunks = hs.data_ptr();
   a.initial_state = nullptr;
   at::Tensor h0_aligned;
   if (h0.has_value()) {

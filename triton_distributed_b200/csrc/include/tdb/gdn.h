@@ -37,7 +37,7 @@ struct GdnChunkArgs {
   void* w;                    // scratch bf16 [NC, H, 64, 128]
   void* kd;                   // scratch bf16 [NC, H, 128, 64]
   void* u;                    // scratch bf16 [NC, H, 64, V]
-  void* v_new;                // scratch bf16 [NC, H, 64, V]
+  void* v_new;                // scratch bf16 [NC, H, 64, V], may be u: a CTA writes a chunk's columns after it has fetched them
   void* h_chunks;             // scratch bf16 [NC, H, 128, V]
   const float* initial_state; // fp32 [N, H, 128, V] or null
   float* final_state;         // fp32 [N, H, 128, V] or null
