@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   const int groups = (r1 - r0 + (1 << gshift) - 1) >> gshift;
   const int gcol = g & ((1 << gshift) - 1);      // this lane's column of a group, its weight row lies up_off further
   const int up_off = g >> gshift ? cols : 0;
-  const int steps = max(1, (kv + 3) >> 2);       // steps of 4 vectors (32 elements of K) of a group; K = 0: one that no warp takes
+  const int steps = (kv + 3) >> 2;               // steps of 4 vectors (32 elements of K) of a group
   const int span = warp_span(groups * steps);
   struct Seg {                                   // what is left of this warp's part of a group, and of its span behind st
     int grp, st, end, left;
   };
   Seg cur;
-  cur.left = kv > 0 ? min(span, groups * steps - warp * span) : 0;
+  cur.left = min(span, groups * steps - warp * span);
   cur.grp = warp * span / steps;
   cur.st = warp * span - cur.grp * steps;
   cur.end = min(steps, cur.st + cur.left);
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     if (tid < MP) {
       float tt = 0.f;
       for (int wi = 0; wi < kGemvWarps; ++wi) tt += s_part[wi][tid];
-      s_rstd[tid] = rsqrtf(tt / static_cast<float>(max(p.K, 1)) + p.eps);
+      s_rstd[tid] = rsqrtf(tt / static_cast<float>(p.K) + p.eps);
     }
   } else if (tid < 16) {
     s_rstd[tid] = 1.f;
@@ -302,15 +302,15 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   attn::cp_async_wait<0>();
   __syncthreads();
 
-  // ---- groups that several warps share: sum their parts (of nothing, where K = 0)
+  // ---- groups that several warps share: sum their parts
   const int shown = groups << gshift;
   for (int i = tid; i < shown * p.M; i += kGemvThreads) {
     const int m = i / shown, rr = i - m * shown;                   // consecutive threads -> consecutive columns
     const int gi = rr >> gshift, gr = rr & ((1 << gshift) - 1);
     const int w0 = gi * steps / span, w1 = ((gi + 1) * steps - 1) / span;
-    if (r0 + rr >= r1 || (w0 == w1 && kv > 0)) continue;
+    if (r0 + rr >= r1 || w0 == w1) continue;
     float v = 0.f, up = 0.f;
-    for (int w = w0; w <= w1 && kv > 0; ++w) {
+    for (int w = w0; w <= w1; ++w) {
       const float* part = red + ((2 * w + (w * span <= gi * steps ? 1 : 0)) * 8 + gr) * (8 * NT) + m;
       v += part[0];
       if (p.swiglu) up += part[4 * 8 * NT];
@@ -450,6 +450,12 @@ cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   if (a.swiglu && (a.N % 2 != 0 || a.all_reduce || a.residual != nullptr)) return cudaErrorInvalidValue;
   const int cols = a.swiglu ? a.N / 2 : a.N;
   if (cols == 0) return cudaSuccess;
+  if (a.K == 0) {      // nothing to sum on any rank, no step to divide among the warps: the residual, or zeros
+    const size_t width = static_cast<size_t>(cols) * 2, pitch = static_cast<size_t>(a.ld_out) * 2;
+    if (a.residual == nullptr) return cudaMemset2DAsync(a.out, pitch, 0, width, a.M, stream);
+    if (a.residual == a.out) return cudaSuccess;
+    return cudaMemcpy2DAsync(a.out, pitch, a.residual, static_cast<size_t>(a.ld_res) * 2, width, a.M, cudaMemcpyDeviceToDevice, stream);
+  }
   const int even = (cols + num_ctas - 1) / num_ctas;
   const int rows = a.all_reduce ? (even + 7) & ~7 : even;
   if (a.all_reduce) {
