@@ -14,12 +14,6 @@ constexpr int kBM = 128;           // query rows per tile
 constexpr int kBN = 64;            // KV tokens per block
 constexpr uint64_t kWaitNs = 4000000000ull;
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 struct FwdParams {
   const __nv_bfloat16* q;
   __nv_bfloat16* out;

@@ -48,11 +48,11 @@ TDB_DEVICE float block_reduce_sum(float v, float* red) {
 // For epilogues on accumulators, where the correctly rounded division is a call that nothing else overlaps (one warp per scheduler: it
 // took eight of the twelve microseconds of a 128 x 256 tile of K = 2048).  The exponential's error grows with its argument, 2 + 1.2 |z| ulp
 // of fp32, the division adds two: 2^-17 of the value at |z| = 88, of which the rounding to bf16 that follows (2^-9) leaves nothing.
-// The exponent is never positive, so that the denominator stays in [1, 2]: with e^-z it left the range of __fdividef, which gives
-// zero for denominators beyond 2^126 (z < -87.3).
+// z / (1 + e^-z) with both sides times 2^-8: __fdividef gives zero for denominators beyond 2^126, so without the factor every z < -87.3;
+// with it z < -92.9, where what is left is no normal number of bf16.
 TDB_DEVICE float silu_f32(float z) {
-  const float e = __expf(-fabsf(z));
-  return __fdividef(z < 0.f ? z * e : z, 1.f + e);
+  constexpr float kScale = 1.f / 256.f;
+  return __fdividef(z * kScale, kScale + ex2(fmaf(z, -1.4426950408889634f, -8.f)));
 }
 TDB_DEVICE float sigmoid_f32(float z) { return 1.f / (1.f + expf(-z)); }
 TDB_DEVICE float gelu_tanh_f32(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
